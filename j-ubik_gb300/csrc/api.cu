@@ -13,6 +13,7 @@
 
 #include "internal.h"
 #include "jubik_common.cuh"
+#include "sep.h"
 
 namespace jubik {
 
@@ -272,6 +273,13 @@ struct jubik_plan {
   void* zs = nullptr;
   void* zu = nullptr;
   int zu_modules = 0;
+  // separable path (sep.h): the entry points of this plan run its row and column
+  // kernels; a fused plan's other buffers then serve grouped launches only
+  bool sep = false;
+  void* sky_rows = nullptr;
+  void* fwd_slabs = nullptr;
+  void* img_rows = nullptr;
+  void* grad_slabs = nullptr;
   // state
   bool psf_set = false, exposure_set = false, data_set = false, lam_valid = false;
   // bumped whenever a buffer address or the readout map that a group copied in
@@ -293,6 +301,12 @@ struct jubik_plan {
     allocs.push_back(*p);
     bytes += n;
     return JUBIK_OK;
+  }
+  // frees the allocations made since `mark` (a size of allocs)
+  void release_from(size_t mark, size_t bytes_then) {
+    for (size_t i = mark; i < allocs.size(); ++i) cudaFree(allocs[i]);
+    allocs.resize(mark);
+    bytes = bytes_then;
   }
   ~jubik_plan() {
     for (int i = 0; i < JUBIK_PHASES; ++i) {
@@ -374,13 +388,6 @@ int adj_terms_log2(const Geom& g) {
   return terms_log2(per * per * g.M);
 }
 
-// row pass of the unfused path's 2-D transforms over batch P x P arrays
-template <typename T>
-int plain_rows(jubik_plan* p, void* data, int64_t batch, bool inverse, cudaStream_t s) {
-  const int64_t P = p->g.P;
-  return fft_batched<T>(p->fft, data, batch * P, (int)P, P * P, P, 1, inverse, 1.0, s);
-}
-
 int do_forward(jubik_plan* p, const void* x, void* out, void* out_lo, double scale,
                cudaStream_t s, void* also_zero = nullptr, int64_t also_zero_bytes = 0,
                bool* zeroed = nullptr, SkyView view = SkyView()) {
@@ -400,7 +407,6 @@ int do_forward(jubik_plan* p, const void* x, void* out, void* out_lo, double sca
   if (p->path == JUBIK_PATH_FUSED) {
     FusedLaunch a{x, out, p->hmain, p->hnyq, p->tw, p->wt, scale, p->spec};
     a.pdl = p->pdl;
-    a.fwd_run = p->fwd_run;
     a.in_ps = view.ps;
     a.in_rs = view.rs;
     a.in_exp = view.exp;
@@ -447,24 +453,6 @@ int do_forward(jubik_plan* p, const void* x, void* out, void* out_lo, double sca
   }
   Phase ph(p, 0, s);
   const bool f32 = p->dtype == JUBIK_F32;
-  if (plain_cols_supported(g.P)) {
-    // row pass over the weighted sky windows; per module chunk: column stage
-    // with the PSF product, inverse row pass, overlap gather
-    const void* tw = f32 ? p->fft.tw32 : p->fft.tw64;
-    JUBIK_TRY(f32 ? fft_rows_windows<float>(p->fft, g, x, false, p->wt, 0, 1, p->zs, s)
-                  : fft_rows_windows<double>(p->fft, g, x, false, p->wt, 0, 1, p->zs, s));
-    for (int m0 = 0; m0 < g.M; m0 += p->zu_modules) {
-      const int nm = std::min(p->zu_modules, g.M - m0);
-      JUBIK_TRY(f32 ? plain_cols_forward<float>(g, p->zs, p->hfull, tw, m0, nm, p->zu, s)
-                    : plain_cols_forward<double>(g, p->zs, p->hfull, tw, m0, nm, p->zu, s));
-      const int64_t batch = (int64_t)nm * plain_pairs(g);
-      JUBIK_TRY(f32 ? plain_rows<float>(p, p->zu, batch, true, s)
-                    : plain_rows<double>(p, p->zu, batch, true, s));
-      JUBIK_TRY(f32 ? plain_overlap_gather<float>(g, p->zu, m0, nm, scale, out, s)
-                    : plain_overlap_gather<double>(g, p->zu, m0, nm, scale, out, s));
-    }
-    return JUBIK_OK;
-  }
   JUBIK_TRY(f32 ? plain_sky_patches<float>(g, x, p->wt, p->zs, s)
                 : plain_sky_patches<double>(g, x, p->wt, p->zs, s));
   JUBIK_TRY(f32 ? fft2_batched<float>(p->fft, p->fft, p->zs, plain_pairs(g), false, s)
@@ -540,26 +528,6 @@ int do_adjoint(jubik_plan* p, const void* cot, void* out_x, void* out_lo, double
   }
   Phase ph(p, 1, s);
   const bool f32 = p->dtype == JUBIK_F32;
-  if (plain_cols_supported(g.P)) {
-    // per module chunk: row pass over the cotangent windows, column stage summing
-    // the conjugate-PSF products over modules; then the inverse row pass and the
-    // gradient gather
-    const void* tw = f32 ? p->fft.tw32 : p->fft.tw64;
-    for (int m0 = 0; m0 < g.M; m0 += p->zu_modules) {
-      const int nm = std::min(p->zu_modules, g.M - m0);
-      const bool first = m0 == 0, last = m0 + nm == g.M;
-      JUBIK_TRY(f32 ? fft_rows_windows<float>(p->fft, g, cot, true, nullptr, m0, nm, p->zu, s)
-                    : fft_rows_windows<double>(p->fft, g, cot, true, nullptr, m0, nm, p->zu, s));
-      JUBIK_TRY(f32 ? plain_cols_adjoint<float>(g, p->zu, p->hfull, tw, m0, nm, first, last,
-                                                p->zs, s)
-                    : plain_cols_adjoint<double>(g, p->zu, p->hfull, tw, m0, nm, first, last,
-                                                 p->zs, s));
-    }
-    JUBIK_TRY(f32 ? plain_rows<float>(p, p->zs, plain_pairs(g), true, s)
-                  : plain_rows<double>(p, p->zs, plain_pairs(g), true, s));
-    return f32 ? plain_grad_gather<float>(g, p->zs, p->wt, scale, out_x, s)
-               : plain_grad_gather<double>(g, p->zs, p->wt, scale, out_x, s);
-  }
   for (int m0 = 0; m0 < g.M; m0 += p->zu_modules) {
     const int nm = std::min(p->zu_modules, g.M - m0);
     JUBIK_TRY(f32 ? plain_cot_patches<float>(g, cot, m0, nm, p->zu, s)
@@ -581,6 +549,112 @@ int finish_words(jubik_plan* p, void* hi, const void* lo, int64_t n, cudaStream_
   if (p->path != JUBIK_PATH_FUSED) return JUBIK_OK;
   return p->dtype == JUBIK_F32 ? combine_words<float>(hi, lo, n, p->pdl, s)
                                : combine_words<double>(hi, lo, n, p->pdl, s);
+}
+
+// Forward of the separable path: sky rows, columns, image rows handed to `mode`
+// (onward: and on to the row spectra of the rows the adjoint starts from).
+int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMode mode, void* out,
+                bool onward, double* energy, cudaStream_t s) {
+  const Geom& g = p->g;
+  SepCols c;
+  c.rows = p->sky_rows;
+  c.hmain = p->hmain;
+  c.hnyq = p->hnyq;
+  c.tw = p->tw;
+  c.wt = p->wt;
+  c.slab = p->fwd_slabs;
+  // (runs exist on module-shared plans, which hold the sky spectra)
+  const int run = p->spec ? fused_fwd_run_len(g, p->dtype, p->fwd_run) : 1;
+  if (run > 1 && sep_run_fits(g, p->dtype, run)) c.run = run;
+  {
+    Phase ph(p, 4, s);
+    SepRows r;
+    r.in = x;
+    r.in_rs = view.rs > 0 ? view.rs : g.ny;
+    r.in_ps = view.ps > 0 ? view.ps : g.pixels();
+    r.in_exp = view.exp ? 1 : 0;
+    r.rows = p->sky_rows;
+    r.tw = p->tw;
+    r.wt = p->wt;
+    r.planes = g.E;
+    JUBIK_TRY(sep_rows(g, p->dtype, SEP_SKY, r, p->pdl, s));
+  }
+  {
+    Phase ph(p, 0, s);
+    JUBIK_TRY(sep_cols(g, p->dtype, SEP_COLS_FWD, c, p->pdl, s));
+  }
+  Phase ph(p, 2, s);
+  SepRows r;
+  r.slab = p->fwd_slabs;
+  r.slab_run = c.run;
+  r.rows = onward ? p->img_rows : nullptr;
+  r.out = out;
+  r.tw = p->tw;
+  r.wt = p->wt;
+  r.eps = p->eps;
+  r.dimg = p->dimg;
+  r.ridx = p->ridx;
+  r.wts = p->wts;
+  r.partials = p->partials;
+  r.counter = p->counter;
+  r.energy = energy;
+  r.scale = scale;
+  r.planes = g.M * g.E;
+  // after the run kernel the rows are launched in full: their looping grid, placed
+  // early between its last long CTAs, took 570 us instead of 334 us (1024^2 x 7 x 3)
+  return sep_rows(g, p->dtype, mode, r, p->pdl && c.run == 1, s);
+}
+
+// Adjoint of the separable path from the row spectra in img_rows.
+int sep_adjoint(jubik_plan* p, void* out_x, double scale, cudaStream_t s) {
+  const Geom& g = p->g;
+  {
+    Phase ph(p, 1, s);
+    SepCols c;
+    c.rows = p->img_rows;
+    c.hmain = p->hmain;
+    c.hnyq = p->hnyq;
+    c.tw = p->tw;
+    c.wt = p->wt;
+    c.slab = p->grad_slabs;
+    JUBIK_TRY(sep_cols(g, p->dtype, SEP_COLS_ADJ, c, p->pdl, s));
+  }
+  Phase ph(p, 5, s);
+  SepRows r;
+  r.slab = p->grad_slabs;
+  r.out = out_x;
+  r.tw = p->tw;
+  r.wt = p->wt;
+  r.scale = scale;
+  r.planes = g.E;
+  return sep_rows(g, p->dtype, SEP_GRAD, r, p->pdl, s);
+}
+
+// Adjoint of an (M, E, nx, ny) image (SEP_COT) or a readout vector (SEP_COT_READOUT).
+int sep_adjoint_of(jubik_plan* p, const void* cot, SepMode mode, void* out_x, double scale,
+                   cudaStream_t s) {
+  {
+    Phase ph(p, 2, s);
+    SepRows r;
+    r.in = cot;
+    r.rows = p->img_rows;
+    r.tw = p->tw;
+    r.wt = p->wt;
+    r.eps = p->eps;
+    r.ridx = p->ridx;
+    r.planes = p->g.M * p->g.E;
+    JUBIK_TRY(sep_rows(p->g, p->dtype, mode, r, p->pdl, s));
+  }
+  return sep_adjoint(p, out_x, scale, s);
+}
+
+// Results of fused plans are 16-byte aligned on every path (as combine_words asks).
+int sep_aligned(const jubik_plan* p, const void* out) {
+  if (p->path == JUBIK_PATH_FUSED && (reinterpret_cast<uintptr_t>(out) & 15)) {
+    set_error("result buffers of a fused plan must be 16-byte aligned");
+    return JUBIK_ERR_INVALID_ARGUMENT;
+  }
+  return JUBIK_OK;
 }
 
 int need(bool ok, const char* what) {
@@ -705,9 +779,23 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
   }
   if ((st = fft1d_init(&p->fft, g.P))) return fail(st);
   p->tw = p->dtype == JUBIK_F32 ? p->fft.tw32 : p->fft.tw64;
+  // the separable kernels where they cover the FFT side and their scratch fits
+  if (d->path != JUBIK_PATH_FUSED_UNIT && sep_supported(g, d->dtype)) {
+    const SepSizes z = sep_sizes(g, d->dtype);
+    const size_t mark = p->allocs.size(), bytes = p->bytes;
+    p->sep = !p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz) &&
+             !p->alloc(&p->hnyq, (size_t)units * g.P * csz) &&
+             !p->alloc(&p->sky_rows, z.sky_rows) && !p->alloc(&p->fwd_slabs, z.fwd_slabs) &&
+             !p->alloc(&p->img_rows, z.img_rows) && !p->alloc(&p->grad_slabs, z.grad_slabs);
+    if (!p->sep) {  // not enough memory: the paths with less scratch
+      cudaGetLastError();
+      p->release_from(mark, bytes);
+      p->hmain = p->hnyq = nullptr;
+    }
+  }
   if (p->path == JUBIK_PATH_FUSED) {
-    if ((st = p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz))) return fail(st);
-    if ((st = p->alloc(&p->hnyq, (size_t)units * g.P * csz))) return fail(st);
+    if (!p->sep && (st = p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz))) return fail(st);
+    if (!p->sep && (st = p->alloc(&p->hnyq, (size_t)units * g.P * csz))) return fail(st);
     if (share && (st = p->alloc(&p->spec, fused_spec_bytes(g, p->dtype)))) return fail(st);
     if (share && (st = p->alloc(&p->acc, fused_spec_bytes(g, p->dtype)))) return fail(st);
     if (share && (st = cuda_status(cudaMemset(p->acc, 0, fused_spec_bytes(g, p->dtype)),
@@ -733,7 +821,7 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
     if ((st = p->alloc(&p->bnd_a, sizeof(uint64_t) *
                                       std::max<int64_t>(energy_partials_count(), kMaxBoundBlocks))))
       return fail(st);
-  } else {
+  } else if (!p->sep) {
     if ((st = p->alloc(&p->hfull, (size_t)units * g.P * (g.P / 2 + 1) * csz))) return fail(st);
     if ((st = p->alloc(&p->zs, (size_t)plain_pairs(g) * g.P * g.P * csz))) return fail(st);
     // bound the per-chunk unit buffer to ~2 GiB; JUBIK_PLAIN_CHUNK_MODULES, when
@@ -747,15 +835,18 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
     p->zu_modules = (int)std::max<size_t>(1, chunk);
     if ((st = p->alloc(&p->zu, per_module * p->zu_modules))) return fail(st);
   }
-  if ((st = p->alloc(&p->conv, img * p->esz))) return fail(st);
-  if ((st = p->alloc(&p->conv_v, img * p->esz))) return fail(st);
-  if ((st = p->alloc(&p->resid, img * p->esz))) return fail(st);
+  if (!p->sep || p->path == JUBIK_PATH_FUSED) {  // (a separable plan never stores these images)
+    if ((st = p->alloc(&p->conv, img * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->conv_v, img * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->resid, img * p->esz))) return fail(st);
+  }
   if ((st = p->alloc(&p->wts, img * p->esz))) return fail(st);
   if ((st = p->alloc(&p->xsky, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
   if ((st = p->alloc(&p->xgrad, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
   if ((st = p->alloc((void**)&p->ridx, img * sizeof(int32_t)))) return fail(st);
   if ((st = p->alloc((void**)&p->rlist, img * sizeof(int64_t)))) return fail(st);
-  if ((st = p->alloc((void**)&p->partials, 2 * energy_partials_count() * sizeof(double))))
+  if ((st = p->alloc((void**)&p->partials,
+                     2 * std::max(energy_partials_count(), kSepMaxBlocks) * sizeof(double))))
     return fail(st);
   if ((st = p->alloc((void**)&p->counter, sizeof(unsigned int)))) return fail(st);
   if ((st = cuda_status(cudaMemset(p->counter, 0, sizeof(unsigned int)), "memset counter")))
@@ -1008,6 +1099,10 @@ int jubik_psf_forward(jubik_plan* p, const void* x, void* out, void* stream) {
   JUBIK_TRY(check_plan(p));
   JUBIK_TRY(need(p->psf_set, "PSF"));
   cudaStream_t s = S(stream);
+  if (p->sep) {
+    JUBIK_TRY(sep_aligned(p, out));
+    return sep_forward(p, x, SkyView(), 1.0, SEP_IMAGE, out, false, nullptr, s);
+  }
   JUBIK_TRY(do_forward(p, x, out, p->conv_lo, 1.0, s));
   return finish_words(p, out, p->conv_lo, image_elems(p), s);
 }
@@ -1017,6 +1112,10 @@ int jubik_psf_adjoint(jubik_plan* p, const void* cot, void* out_x, void* stream)
   JUBIK_TRY(check_plan(p));
   JUBIK_TRY(need(p->psf_set, "PSF"));
   cudaStream_t s = S(stream);
+  if (p->sep) {
+    JUBIK_TRY(sep_aligned(p, out_x));
+    return sep_adjoint_of(p, cot, SEP_COT, out_x, 1.0, s);
+  }
   JUBIK_TRY(do_adjoint(p, cot, out_x, p->grad_lo, 1.0, s));
   return finish_words(p, out_x, p->grad_lo, (int64_t)p->g.E * p->g.pixels(), s);
 }
@@ -1026,6 +1125,9 @@ int jubik_response_forward(jubik_plan* p, const void* x, void* out_readout, void
   JUBIK_TRY(check_plan(p));
   JUBIK_TRY(need(p->psf_set, "PSF"));
   cudaStream_t s = S(stream);
+  if (p->sep)
+    return sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_READOUT, out_readout, false,
+                       nullptr, s);
   JUBIK_TRY(do_forward(p, x, p->conv, p->conv_lo, p->desc.pixel_area, s));
   const void* lo = p->path == JUBIK_PATH_FUSED ? p->conv_lo : nullptr;
   Phase ph(p, 2, s);
@@ -1046,6 +1148,10 @@ int jubik_response_vjp(jubik_plan* p, const void* cot_readout, void* out_x, void
   JUBIK_TRY(check_plan(p));
   JUBIK_TRY(need(p->psf_set, "PSF"));
   cudaStream_t s = S(stream);
+  if (p->sep) {
+    JUBIK_TRY(sep_aligned(p, out_x));
+    return sep_adjoint_of(p, cot_readout, SEP_COT_READOUT, out_x, p->desc.pixel_area, s);
+  }
   {
     Phase ph(p, 2, s);
     JUBIK_TRY_CUDA(cudaMemsetAsync(p->resid, 0, image_elems(p) * p->esz, s));
@@ -1066,6 +1172,13 @@ int jubik_poisson_energy_grad(jubik_plan* p, const void* x, double* energy, void
   JUBIK_TRY(need(p->psf_set, "PSF"));
   JUBIK_TRY(need(p->data_set, "data"));
   cudaStream_t s = S(stream);
+  if (p->sep) {
+    if (grad_x) JUBIK_TRY(sep_aligned(p, grad_x));
+    JUBIK_TRY(sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_LIKE, nullptr,
+                          grad_x != nullptr, energy, s));
+    p->lam_valid = true;
+    return grad_x ? sep_adjoint(p, grad_x, p->desc.pixel_area, s) : JUBIK_OK;
+  }
   bool grad_zeroed = false;
   JUBIK_TRY(do_forward(p, x, p->conv, p->conv_lo, p->desc.pixel_area, s, grad_x,
                        (int64_t)p->g.E * p->g.pixels() * (int64_t)p->esz, &grad_zeroed));
@@ -1107,6 +1220,14 @@ int jubik_poisson_energy_grad_logsky(jubik_plan* p, const void* s_log, int32_t e
   view.rs = ny_pad;
   view.ps = (int64_t)nx_pad * ny_pad;
   view.exp = true;
+  const void* glo = nullptr;
+  if (p->sep) {
+    JUBIK_TRY(sep_forward(p, s_log, view, p->desc.pixel_area, SEP_LIKE, nullptr,
+                          grad_s != nullptr, energy, s));
+    p->lam_valid = true;
+    if (!grad_s) return JUBIK_OK;
+    JUBIK_TRY(sep_adjoint(p, p->xgrad, p->desc.pixel_area, s));
+  } else {
   bool grad_zeroed = false;
   JUBIK_TRY(do_forward(p, s_log, p->conv, p->conv_lo, p->desc.pixel_area, s,
                        grad_s ? p->xgrad : nullptr, (int64_t)g.E * g.pixels() * (int64_t)p->esz,
@@ -1128,7 +1249,8 @@ int jubik_poisson_energy_grad_logsky(jubik_plan* p, const void* s_log, int32_t e
   if (!grad_s) return JUBIK_OK;
   JUBIK_TRY(do_adjoint(p, p->resid, p->xgrad, p->grad_lo, p->desc.pixel_area, s, grad_zeroed,
                        energy_partials_count()));
-  const void* glo = p->path == JUBIK_PATH_FUSED ? p->grad_lo : nullptr;
+  glo = p->path == JUBIK_PATH_FUSED ? p->grad_lo : nullptr;
+  }
   const int64_t n = (int64_t)e_pad * nx_pad * ny_pad;
   if (p->dtype == JUBIK_F32)
     k_logsky_grad<float><<<blocks_for(n), 256, 0, s>>>((const float*)s_log,
@@ -1149,6 +1271,18 @@ int jubik_metric_apply(jubik_plan* p, const void* x, const void* v, void* out, v
   JUBIK_TRY(need(p->psf_set, "PSF"));
   cudaStream_t s = S(stream);
   const int64_t img = image_elems(p);
+  if (p->sep) {
+    JUBIK_TRY(sep_aligned(p, out));
+    if (x) {
+      JUBIK_TRY(sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_WEIGHTS, nullptr, false,
+                            nullptr, s));
+      p->lam_valid = true;
+    }
+    JUBIK_TRY(need(p->lam_valid, "lambda (call with x or after poisson_energy_grad)"));
+    JUBIK_TRY(sep_forward(p, v, SkyView(), p->desc.pixel_area, SEP_METRIC, nullptr, true, nullptr,
+                          s));
+    return sep_adjoint(p, out, p->desc.pixel_area, s);
+  }
   const bool two = p->path == JUBIK_PATH_FUSED;
   if (x) {  // weights eps^2 / lam of a new lam = R(x), as the likelihood pass leaves them
     JUBIK_TRY(do_forward(p, x, p->conv, p->conv_lo, p->desc.pixel_area, s));

@@ -5,6 +5,7 @@
 
 #include "fft_codelets.cuh"
 #include "internal.h"
+#include "likelihood.cuh"
 
 namespace jubik {
 
@@ -520,94 +521,13 @@ __global__ void k_readout_scatter(const T* __restrict__ vec, const T* __restrict
 
 // --------------------------------------------------------------- Poisson
 // Compensated (Kahan) accumulation in the working precision per thread, FP64
-// across threads and blocks; the last block sums the block partials in a
-// fixed order, so the total is deterministic.
-template <typename T>
-struct Kahan {
-  T s = (T)0, c = (T)0;
-  __device__ __forceinline__ void add(T v) {
-    const T y = v - c;
-    const T t = s + y;
-    c = (t - s) - y;
-    s = t;
-  }
-  __device__ __forceinline__ double value() const { return (double)s - (double)c; }
-};
-
-// Block sums of (a, b) into partials[bid]; the last of nblocks blocks to finish
-// sums the partials in a fixed order (deterministic) and writes a - b.
-__device__ __forceinline__ void block_reduce2_of(double a, double b, double* partials,
-                                                 unsigned int* counter, double* energy,
-                                                 unsigned int bid, unsigned int nblocks) {
-  __shared__ double sa[kBlock], sb[kBlock];
-  __shared__ bool last;
-  sa[threadIdx.x] = a;
-  sb[threadIdx.x] = b;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      sa[threadIdx.x] += sa[threadIdx.x + w];
-      sb[threadIdx.x] += sb[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    partials[2 * bid] = sa[0];
-    partials[2 * bid + 1] = sb[0];
-    __threadfence();
-    const unsigned int done = atomicAdd(counter, 1u);
-    last = (done == nblocks - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  // the last block sums the block partials in a fixed order (deterministic)
-  __threadfence();
-  double p1 = 0.0, p2 = 0.0;
-  for (unsigned int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-    p1 += __ldcg(partials + 2 * i);
-    p2 += __ldcg(partials + 2 * i + 1);
-  }
-  sa[threadIdx.x] = p1;
-  sb[threadIdx.x] = p2;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      sa[threadIdx.x] += sa[threadIdx.x + w];
-      sb[threadIdx.x] += sb[threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    // H = sum(lam) - vdot(d, log(lam))
-    if (energy) energy[0] = sa[0] - sb[0];
-    *counter = 0u;
-  }
-}
-
+// across threads and blocks (likelihood.cuh); the last block sums the block
+// partials in a fixed order, so the total is deterministic.
 __device__ __forceinline__ void block_reduce2(double a, double b, double* partials,
-                                              unsigned int* counter, double* energy) {
-  block_reduce2_of(a, b, partials, counter, energy, blockIdx.x, gridDim.x);
-}
-
-// One pass over the (M,E,nx,ny) images: lam = eps * conv where a pixel is read
-// out (count image >= 0), the energy terms, the residual eps * (1 - d/lam)
-// (0 elsewhere) and, optionally, the metric weight eps^2 / lam (0 elsewhere)
-// that later Fisher-metric products apply to R v: the image-space weights of
-// R^T diag(1/lam) R (the exposure enters once from R and once from R^T).
-template <typename T>
-__device__ __forceinline__ void poisson_px(T conv, T ep, int32_t d, T& w_o, T& res_o,
-                                           Kahan<T>& s_lam, Kahan<T>& s_dlog) {
-  if (d < 0) {
-    res_o = (T)0;
-    w_o = (T)0;
-    return;
-  }
-  const T lam = ep * conv;
-  const T dd = (T)d;
-  s_lam.add(lam);
-  s_dlog.add(dd * log(lam));
-  w_o = (ep * ep) / lam;
-  res_o = ep * ((T)1 - dd / lam);
+                                              unsigned int* counter, double* energy,
+                                              unsigned int bid, unsigned int nblocks) {
+  __shared__ double sa[kBlock], sb[kBlock];
+  block_reduce2_of(a, b, sa, sb, partials, counter, energy, bid, nblocks);
 }
 
 // Block maximum of per-thread magnitudes (float or double bits; a NaN sorts
@@ -715,7 +635,7 @@ __device__ __forceinline__ void poisson_image_body(const T* __restrict__ conv,
     if (rmax) mr.add(r);
   }
   if (rmax) store_block_max(mr.bits(), rmax, bid);
-  block_reduce2_of(s_lam.value(), s_dlog.value(), partials, counter, energy, bid, nblocks);
+  block_reduce2(s_lam.value(), s_dlog.value(), partials, counter, energy, bid, nblocks);
 }
 
 template <typename T>
@@ -897,7 +817,7 @@ __global__ void __launch_bounds__(kBlock)
     s_dlog.add(d * log(l));
     if (grad) grad[i] = (T)1 - d / l;
   }
-  block_reduce2(s_lam.value(), s_dlog.value(), partials, counter, energy);
+  block_reduce2(s_lam.value(), s_dlog.value(), partials, counter, energy, blockIdx.x, gridDim.x);
 }
 
 // Metric weights eps^2 / lam of a fresh lam = eps * conv (conv in two words,

@@ -1,0 +1,599 @@
+// Row kernels of the separable response (see sep.h).
+//
+// A CTA takes one or more pairs of image rows (2t, 2t + 1) of one plane with
+// all n windows (patch columns) that cut them.  The two real rows of a pair
+// travel as the real and imaginary part of one complex sequence per window.
+//   inverse half: slabs -> row spectra of the pair (sum over the slabs that
+//     cover the row, in order) -> inverse transforms -> overlap-add over the
+//     windows in shared memory (window order, compensated) -> image rows;
+//   pixels: likelihood, metric weights, readout, gradient, ...;
+//   forward half: image rows -> windows -> transforms -> row spectra.
+// Both halves run in one kernel for the likelihood and the metric, so the image
+// of expected counts is never stored.
+//
+// Each transform of side P = 16 L1 is a two-phase four-step in place: slots
+// 16 cls + q lie at 17 cls + q (the odd class pitch spreads both the
+// class-parallel and the slot-parallel accesses over the banks).  A warp takes two
+// sequences through all of its phases -- load and join of the two rows' spectra,
+// DFT-L1 (16 classes x 2 sequences: one per lane), DFT-16; and back -- with warp
+// barriers only; the CTA meets twice per item, before and after the overlap-add.
+// The kernels are bound by the latency of the spectrum loads and by instruction
+// issue; warps that drift apart overlap the one with the other.
+#include "likelihood.cuh"
+#include "sep_dev.cuh"
+
+namespace jubik {
+namespace {
+
+struct RowK {
+  SepRows a;
+  int mode;
+  int nx, ny, n, dx, half, margin, sr_max, sc_max, K;
+  int nslab, step, height;   // slabs of a patch column: start every step rows, height rows
+  int late;                  // rows the last slab starts before its stride (clamped windows)
+  int few;                   // at most 4 windows cover a column, all in buf, none clamped
+  int seqs;                  // sequences (row pair x window) in shared memory at once
+  int rp;                    // row pairs per item
+  int per;                   // items per plane
+  int items;                 // items in all
+  uint32_t mul_dx, mul_step;  // floor(u / d) = high word of u mul (row_div)
+  uint32_t div_per;
+  float scale32;
+  double scale64;
+};
+template <typename T> __device__ __forceinline__ T row_scale(const RowK& k);
+template <> __device__ __forceinline__ float row_scale<float>(const RowK& k) { return k.scale32; }
+template <> __device__ __forceinline__ double row_scale<double>(const RowK& k) {
+  return k.scale64;
+}
+
+// Sequences (row pair x window) a CTA holds at once: 16, or as many as fit beside
+// the image rows of a wide field (row_seqs).
+constexpr int kRowSeqs = 16;
+
+template <int L1>
+constexpr int row_pitch() { return 17 * L1 + (L1 % 16 == 0 ? 8 : 0); }
+constexpr int kRowThreads = 16 * kRowSeqs;  // two sequences a warp
+// CTAs per SM the register budget is cut for: 80 registers (FP32), 128 for the
+// long DFT-L1 of P >= 320 and for FP64, 255 for both
+template <typename T, int L1>
+constexpr int row_ctas() { return sizeof(T) == 4 ? (L1 <= 16 ? 3 : 2) : (L1 <= 16 ? 2 : 1); }
+constexpr int kRowTw = 18;  // pitch of a class's twiddles (16-byte pairs)
+
+// bytes of dynamic shared memory: sequences, twiddles by class, image rows (and,
+// with more windows than sequences, the overlap-add's compensation), windows by column
+template <typename T, int L1>
+size_t row_smem(int n, int ny, int rp, int most) {
+  const size_t seqs = (size_t)std::min(most, n * rp) * row_pitch<L1>();
+  const size_t lines = (size_t)rp * ny * (n > most ? 2 : 1);
+  const size_t red = 2 * sizeof(double) * kRowThreads;  // the block sums reuse seqs
+  return std::max(sizeof(cx<T>) * seqs, red) + sizeof(cx<T>) * (lines + kRowTw * L1) +
+         sizeof(uint32_t) * ny;
+}
+inline int row_pairs(int n, int nx, int most) {  // row pairs of an item
+  return std::min(std::max(1, most / n), (nx + 1) / 2);
+}
+// the most sequences (of 16, 8, 4, 2) that fit beside the rows of this field; 0: none
+template <typename T, int L1>
+int row_seqs(const Geom& g) {
+  for (int most = kRowSeqs; most >= 2; most /= 2)
+    if (row_smem<T, L1>(g.n, g.ny, row_pairs(g.n, g.nx, most), most) + 1024 <=
+        (size_t)max_smem_optin())
+      return most;
+  return 0;
+}
+
+// floor(u / d) for 0 <= u by the multiply-high constant of d >= 2 (mulhi_divisor)
+__device__ __forceinline__ int row_div(int u, uint32_t mul) { return (int)__umulhi((uint32_t)u, mul); }
+__device__ __forceinline__ int row_slot(int z) { return (z >> 4) * 17 + (z & 15); }
+
+// twiddles q and q + 1 (q even) of a class in one 16-byte load (FP32)
+__device__ __forceinline__ void row_twiddles(const float2* tw, int q, float2& a, float2& b) {
+  const float4 t = *reinterpret_cast<const float4*>(tw + q);
+  a = make_float2(t.x, t.y);
+  b = make_float2(t.z, t.w);
+}
+__device__ __forceinline__ void row_twiddles(const double2* tw, int q, double2& a, double2& b) {
+  a = tw[q];
+  b = tw[q + 1];
+}
+
+// DFT-L1 of class `ca` of a sequence, in place
+template <typename T, int L1, bool INV>
+__device__ __forceinline__ void row_dft_l1(cx<T>* seq, int ca) {
+  cx<T>* row = seq + ca;
+  cx<T> v[L1];
+#pragma unroll
+  for (int i = 0; i < L1; ++i) v[i] = row[17 * i];
+  Dft<L1, INV, T>::run(v);
+#pragma unroll
+  for (int i = 0; i < L1; ++i) row[17 * i] = v[i];
+}
+
+// MODE: what happens to the pixels (SEP_IMAGE also serves SEP_READOUT and
+// SEP_WEIGHTS, by a.mode; SEP_COT also SEP_COT_READOUT).  FWD: transform the rows
+// that result.
+template <typename T, int L1, int MODE, bool FWD>
+__global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(RowK k) {
+  constexpr int P = 16 * L1, H = P / 2, WP = row_pitch<L1>();
+  constexpr bool INV = MODE != SEP_SKY && MODE != SEP_COT, GRAD = MODE == SEP_GRAD;
+  // sequences whose DFT-16 items a warp runs at once (L1 lanes each)
+  constexpr int SEQ16 = 2 * L1 <= 32 ? 2 : 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const SepRows& a = k.a;
+  const int n = k.n, ny = k.ny, nx = k.nx;
+  const int nsq = min(k.seqs, n * k.rp);
+  const size_t seq_bytes = max(sizeof(cx<T>) * (size_t)(nsq * WP), 2 * sizeof(double) * kRowThreads);
+  cx<T>* buf = reinterpret_cast<cx<T>*>(smem_raw);
+  cx<T>* stw = reinterpret_cast<cx<T>*>(smem_raw + seq_bytes);
+  cx<T>* line = stw + kRowTw * L1;
+  cx<T>* comp = line + (size_t)k.rp * ny;  // n > k.seqs only
+  uint32_t* xwin = reinterpret_cast<uint32_t*>(line + (size_t)k.rp * ny * (n > k.seqs ? 2 : 1));
+  const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31;
+  const int q0 = 2 * (tid >> 5);          // this warp's sequences: q0, q0 + 1
+  const int cls = lane % L1, sub = lane / L1;  // this lane's DFT-16 item
+  // slots of kx = lane and of kx = P - lane (32 further on: 34 slots)
+  const int slot_p = row_slot(lane), slot_m = row_slot(P - lane);
+  const T* __restrict__ wt = (const T*)a.wt;
+  const T* __restrict__ eps = (const T*)a.eps;
+  const int off = GRAD ? k.margin : 0;
+  const int base_c = -k.half - k.margin + off;
+  const int wx = GRAD ? k.K : P;  // window columns the overlap-add takes
+  sep_trigger();
+  {
+    const cx<T>* tw = (const cx<T>*)a.tw;
+    for (int i = tid; i < 16 * L1; i += NT) {
+      const int cc = i >> 4, q = i & 15;
+      stw[kRowTw * cc + q] = __ldg(tw + cc * q);
+    }
+  }
+  if (INV) {
+    // the windows that cover column x: the first one and their count
+    for (int x = tid; x < ny; x += NT) {
+      const int d = x - base_c, under = d - wx + 1;
+      int hi = min(n - 1, row_div(d, k.mul_dx));
+      // a last window that starts early (clamped) may cover x too
+      if (hi + 1 == n - 1 && k.sc_max <= d) ++hi;
+      const int lo = under <= 0 ? 0 : row_div(under + k.dx - 1, k.mul_dx);
+      const uint32_t cw = hi >= lo ? (uint32_t)(hi - lo + 1) : 0u;
+      const int xi = d - lo * k.dx;  // x within window lo
+      // few: place of x in window lo, count, xi; else: lo, count
+      if (k.few)
+        xwin[x] = cw ? ((uint32_t)xi << 20 | cw << 16 | (uint32_t)(lo * WP + xi + off)) : 0u;
+      else
+        xwin[x] = cw ? ((uint32_t)lo << 16 | cw) : 0u;
+    }
+  }
+  sep_wait();
+  __syncthreads();
+  const cx<T>* mytw = stw + kRowTw * cls;
+  const T scale = row_scale<T>(k);
+  Kahan<T> s_lam, s_dlog;
+  const int nchunk = (n * k.rp + k.seqs - 1) / k.seqs;  // > 1 only when rp == 1
+
+  for (int item = blockIdx.x; item < k.items; item += gridDim.x) {
+    const int pl = sep_div(item, k.per, k.div_per);
+    const int t0 = (item - pl * k.per) * k.rp;  // first row pair
+    if (INV) {
+      // ---- slabs -> image rows
+      for (int ch = 0; ch < nchunk; ++ch) {
+        const int j0 = ch * k.seqs, jn = min(k.seqs, n - j0);  // windows j0 .. j0 + jn - 1
+        const int cnt = jn * k.rp;                                 // sequences in buf
+        const int hs = k.height * H;
+        // the slabs that cover the pair's rows, in order (a row beyond the field: none):
+        // their number and the row's offset in each
+        int lo[2], m[2], o[2][3], had = -1;
+#pragma unroll 1
+        for (int s = q0; s < q0 + 2 && s < cnt; ++s) {
+          const int r = k.rp == 1 ? 0 : s / jn, j = j0 + s - r * jn;
+          const int row0 = 2 * (t0 + r);
+          if (r != had) {
+            had = r;
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              const int d = row0 + b - base_c, under = d - k.height + 1;
+              int hi = min(k.nslab - 1, row_div(d, k.mul_step));
+              if (hi + 1 == k.nslab - 1 && k.nslab * k.step - k.step - k.late <= d) ++hi;
+              lo[b] = under <= 0 ? 0 : row_div(under + k.step - 1, k.mul_step);
+              m[b] = row0 + b < nx ? hi - lo[b] + 1 : 0;
+#pragma unroll
+              for (int u = 0; u < 3; ++u) {
+                const int i = lo[b] + u;
+                o[b][u] = i * hs + (d - i * k.step + (i == k.nslab - 1 ? k.late : 0)) * H;
+              }
+            }
+          }
+          const cx<T>* p = (const cx<T>*)a.slab + ((int64_t)pl * n + j) * hs * k.nslab + lane;
+          cx<T>* wp = buf + s * WP + slot_p;
+          cx<T>* wm = buf + s * WP + slot_m;
+#pragma unroll
+          for (int t = 0; t < (H + 31) / 32; ++t) {
+            if (H % 32 && lane + 32 * t >= H) break;
+            cx<T> v[2];
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              const cx<T> z = mkc<T>((T)0, (T)0);
+              const cx<T> v0 = 0 < m[b] ? p[o[b][0] + 32 * t] : z;
+              const cx<T> v1 = 1 < m[b] ? p[o[b][1] + 32 * t] : z;
+              const cx<T> v2 = 2 < m[b] ? p[o[b][2] + 32 * t] : z;
+              v[b] = cadd<T>(cadd<T>(v0, v1), v2);
+            }
+            if (max(m[0], m[1]) > 3) {  // margins beyond a stride: more slabs
+#pragma unroll
+              for (int b = 0; b < 2; ++b)
+                for (int u = 3; u < m[b]; ++u) {
+                  const int i = lo[b] + u;
+                  v[b] = cadd<T>(v[b], p[i * hs + (row0 + b - base_c - i * k.step +
+                                                   (i == k.nslab - 1 ? k.late : 0)) * H + 32 * t]);
+                }
+            }
+            // join the two rows (kx = 0: the packed real kx = 0 and kx = P / 2 values)
+            const bool dc = t == 0 && lane == 0;
+            wp[34 * t] = dc ? mkc<T>(v[0].x, v[1].x) : join_p<T>(v[0], v[1]);
+            (dc ? wp + row_slot(H) : wm - 34 * t)[0] =
+                dc ? mkc<T>(v[0].y, v[1].y) : join_m<T>(v[0], v[1]);
+          }
+        }
+        __syncwarp();
+        if (q0 + (lane >> 4) < cnt) row_dft_l1<T, L1, true>(buf + (q0 + (lane >> 4)) * WP, lane & 15);
+        __syncwarp();
+#pragma unroll 1
+        for (int h = 0; h < 2; h += SEQ16) {  // DFT-16 -> natural order
+          const int s = q0 + h + sub;
+          const bool on = sub < SEQ16 && s < cnt;
+          cx<T> v[16];
+          if (on) {
+            const cx<T>* src = buf + s * WP + 17 * cls;
+#pragma unroll
+            for (int q = 0; q < 16; q += 2) {
+              cx<T> wa, wb;
+              row_twiddles(mytw, q, wa, wb);
+              v[q] = q ? cmulc<T>(src[q], wa) : src[q];
+              v[q + 1] = cmulc<T>(src[q + 1], wb);
+            }
+            Dft<16, true, T>::run(v);
+          }
+          __syncwarp();  // in place: every lane has read
+          if (on) {
+            cx<T>* dst = buf + s * WP + cls;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) dst[L1 * q] = v[q];
+          }
+        }
+        __syncthreads();
+        // overlap-add over the windows, in window order, and the pixels
+        const bool last = ch == nchunk - 1;
+        for (int r = 0; r < k.rp; ++r) {
+          const int row0 = 2 * (t0 + r);
+          if (row0 >= nx) break;
+          const int64_t px0 = ((int64_t)pl * nx + row0) * ny;
+          const bool two = row0 + 1 < nx;
+          const cx<T>* wbuf = buf + (r * jn) * WP;
+          constexpr int U = 4;  // columns whose pixel inputs are loaded together
+          for (int xb = tid; xb < ny; xb += U * NT) {
+            T f[U][2];
+            int32_t ix[U][2];
+            if (MODE != SEP_GRAD) {
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                  const int x = xb + u * NT;
+                  const int64_t p = px0 + (int64_t)b * ny + x;
+                  f[u][b] = (T)1;
+                  ix[u][b] = -1;
+                  if (last && x < ny && (b == 0 || two)) {
+                    if (MODE == SEP_LIKE) ix[u][b] = a.dimg[p];
+                    if (MODE == SEP_METRIC) f[u][b] = ((const T*)a.wts)[p];
+                    if (MODE == SEP_IMAGE && k.mode != SEP_IMAGE) ix[u][b] = a.ridx[p];
+                    if (MODE != SEP_METRIC && eps && (MODE == SEP_LIKE || k.mode != SEP_IMAGE))
+                      f[u][b] = eps[p];
+                  }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const int x = xb + u * NT;
+              if (x >= ny) break;
+              const uint32_t e = xwin[x];
+              cx<T> sum;
+              if (k.few) {
+                // compensated sum of up to four windows' values, in window order
+                const cx<T>* w = wbuf + (e & 0xffffu);
+                const int cw = (int)(e >> 16) & 15, S = WP - k.dx;
+                const cx<T> z = mkc<T>((T)0, (T)0);
+                cx<T> z0 = cw > 0 ? w[0] : z, z1 = cw > 1 ? w[S] : z;
+                cx<T> z2 = cw > 2 ? w[2 * S] : z;
+                if (GRAD) {  // the windows' column weights
+                  const T* wx0 = wt + (e >> 20);
+                  const T g0 = cw > 0 ? wx0[0] : (T)0, g1 = cw > 1 ? wx0[-k.dx] : (T)0;
+                  const T g2 = cw > 2 ? wx0[-2 * k.dx] : (T)0;
+                  z0 = mkc<T>(g0 * z0.x, g0 * z0.y);
+                  z1 = mkc<T>(g1 * z1.x, g1 * z1.y);
+                  z2 = mkc<T>(g2 * z2.x, g2 * z2.y);
+                }
+                const cx<T> t = cadd<T>(z0, z1);
+                const cx<T> y = csub<T>(z2, csub<T>(csub<T>(t, z0), z1));
+                sum = cadd<T>(t, y);
+                if (cw > 3) {
+                  cx<T> z3 = w[3 * S];
+                  if (GRAD) {
+                    const T g3 = wt[(int)(e >> 20) - 3 * k.dx];
+                    z3 = mkc<T>(g3 * z3.x, g3 * z3.y);
+                  }
+                  sum = cadd<T>(sum, csub<T>(z3, csub<T>(csub<T>(sum, t), y)));
+                }
+              } else {
+                int j = (int)(e >> 16), jend = j + (int)(e & 0xffffu);
+                j = max(j, j0);
+                jend = min(jend, j0 + jn);
+                Kahan<T> re, im;
+                if (ch > 0) {
+                  const cx<T> s = line[x], cc = comp[x];
+                  re.s = s.x;
+                  im.s = s.y;
+                  re.c = cc.x;
+                  im.c = cc.y;
+                }
+                const cx<T>* w = wbuf + (j - j0) * WP + x + off - base_c;
+                for (int st = j * k.dx; j < jend; ++j, st += k.dx, w += WP) {
+                  const int s0 = min(st, k.sc_max);
+                  cx<T> z = w[-s0];
+                  if (GRAD) {
+                    const T ww = wt[x - base_c - s0];
+                    z = mkc<T>(ww * z.x, ww * z.y);
+                  }
+                  re.add(z.x);
+                  im.add(z.y);
+                }
+                sum = mkc<T>(re.s, im.s);
+                if (!last) {
+                  line[x] = sum;
+                  comp[x] = mkc<T>(re.c, im.c);
+                  continue;
+                }
+              }
+              const T v[2] = {scale * sum.x, scale * sum.y};
+              T o[2] = {(T)0, (T)0};
+#pragma unroll
+              for (int b = 0; b < 2; ++b) {
+                if (b && !two) break;
+                const int64_t p = px0 + (int64_t)b * ny + x;
+                if (MODE == SEP_LIKE) {
+                  T wgt;
+                  poisson_px<T>(v[b], f[u][b], ix[u][b], wgt, o[b], s_lam, s_dlog);
+                  __stcs((T*)a.wts + p, wgt);
+                } else if (MODE == SEP_METRIC) {
+                  o[b] = f[u][b] * v[b];
+                } else if (MODE == SEP_GRAD || k.mode == SEP_IMAGE) {
+                  ((T*)a.out)[p] = v[b];
+                } else if (k.mode == SEP_READOUT) {
+                  if (ix[u][b] >= 0) ((T*)a.out)[ix[u][b]] = eps ? f[u][b] * v[b] : v[b];
+                } else {  // SEP_WEIGHTS
+                  const T ep = f[u][b];
+                  ((T*)a.wts)[p] = ix[u][b] < 0 ? (T)0 : (ep * ep) / (ep * v[b]);
+                }
+              }
+              if (FWD) line[r * ny + x] = mkc<T>(o[0], o[1]);
+            }
+          }
+        }
+        __syncthreads();  // every window has been read, every image row written
+      }
+    } else {
+      // ---- rows of the input
+      for (int r = 0; r < k.rp; ++r) {
+        const int row0 = 2 * (t0 + r);
+        if (row0 >= nx) break;
+        const bool two = row0 + 1 < nx;
+#pragma unroll 2
+        for (int x = tid; x < ny; x += NT) {
+          T o[2] = {(T)0, (T)0};
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            if (b && !two) break;
+            if (MODE == SEP_SKY) {
+              const T v = ((const T*)a.in)[pl * a.in_ps + (int64_t)(row0 + b) * a.in_rs + x];
+              o[b] = a.in_exp ? exp(v) : v;
+            } else {
+              const int64_t p = ((int64_t)pl * nx + row0 + b) * ny + x;
+              if (k.mode == SEP_COT) {
+                o[b] = ((const T*)a.in)[p];
+              } else {  // SEP_COT_READOUT
+                const int32_t i = a.ridx[p];
+                if (i >= 0) {
+                  const T v = ((const T*)a.in)[i];
+                  o[b] = eps ? eps[p] * v : v;
+                }
+              }
+            }
+          }
+          line[r * ny + x] = mkc<T>(o[0], o[1]);
+        }
+      }
+      __syncthreads();
+    }
+    if (FWD) {
+      // ---- image rows -> row spectra of every window
+      for (int ch = 0; ch < nchunk; ++ch) {
+        const int j0 = ch * k.seqs, jn = min(k.seqs, n - j0);
+        const int cnt = jn * k.rp;
+#pragma unroll 1
+        for (int h = 0; h < 2; h += SEQ16) {
+          const int s = q0 + h + sub;
+          if (sub >= SEQ16 || s >= cnt) continue;
+          const int r = k.rp == 1 ? 0 : s / jn;
+          const int j = j0 + s - r * jn;
+          const int x0 = min(j * k.dx, k.sc_max) - k.half - k.margin + cls;
+          const cx<T>* src = line + r * ny + x0;
+          const bool there = 2 * (t0 + r) < nx;
+          cx<T> v[16];
+          if (MODE != SEP_SKY && there && x0 >= 0 && x0 + P - L1 < ny) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = src[L1 * q];
+          } else {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              bool in = there && (unsigned)(x0 + L1 * q) < (unsigned)ny;
+              const int xa = cls + L1 * q - k.margin;
+              // outside the window the value does not enter (it may be infinite)
+              if (MODE == SEP_SKY) in = in && (unsigned)xa < (unsigned)k.K;
+              v[q] = in ? src[L1 * q] : mkc<T>((T)0, (T)0);
+              if (MODE == SEP_SKY) {
+                const T w = in ? wt[xa] : (T)0;
+                v[q] = mkc<T>(w * v[q].x, w * v[q].y);
+              }
+            }
+          }
+          Dft<16, false, T>::run(v);
+          cx<T>* dst = buf + s * WP + 17 * cls;
+#pragma unroll
+          for (int q = 0; q < 16; q += 2) {
+            cx<T> wa, wb;
+            row_twiddles(mytw, q, wa, wb);
+            dst[q] = q ? cmul<T>(v[q], wa) : v[q];
+            dst[q + 1] = cmul<T>(v[q + 1], wb);
+          }
+        }
+        __syncwarp();
+        if (q0 + (lane >> 4) < cnt) row_dft_l1<T, L1, false>(buf + (q0 + (lane >> 4)) * WP, lane & 15);
+        __syncwarp();
+#pragma unroll 1
+        for (int s = q0; s < q0 + 2 && s < cnt; ++s) {  // split into the two rows' spectra
+          const int r = k.rp == 1 ? 0 : s / jn, j = j0 + s - r * jn;
+          const int row0 = 2 * (t0 + r);
+          if (row0 >= nx) break;
+          const bool two = row0 + 1 < nx;
+          cx<T>* dst = (cx<T>*)a.rows + (((int64_t)pl * n + j) * nx + row0) * H + lane;
+          const cx<T>* wp = buf + s * WP + slot_p;
+          const cx<T>* wm = buf + s * WP + slot_m;
+#pragma unroll
+          for (int t = 0; t < (H + 31) / 32; ++t) {
+            if (H % 32 && lane + 32 * t >= H) break;
+            const bool dc = t == 0 && lane == 0;
+            const cx<T> zp = wp[34 * t], zm = (dc ? wp + row_slot(H) : wm - 34 * t)[0];
+            dst[32 * t] = dc ? mkc<T>(zp.x, zm.x) : split_a<T>(zp, zm);
+            if (two) dst[H + 32 * t] = dc ? mkc<T>(zp.y, zm.y) : split_b<T>(zp, zm);
+          }
+        }
+        __syncwarp();  // this warp's sequences have been read
+      }
+      // the image rows have been read (an inverse half meets at its own barrier first)
+      if (!INV) __syncthreads();
+    }
+  }
+  if (MODE == SEP_LIKE) {
+    __syncthreads();
+    double* red = reinterpret_cast<double*>(smem_raw);  // every sequence has been read
+    block_reduce2_of(s_lam.value(), s_dlog.value(), red, red + NT, a.partials, a.counter,
+                     a.energy, blockIdx.x, gridDim.x);
+  }
+}
+
+// bound of the numerators that the kernels divide by dx or a slab's stride
+inline int64_t sep_reach(const Geom& g) { return std::max(g.nx, g.ny) + 4 * (int64_t)g.P; }
+
+template <typename T, int L1, int MODE, bool FWD>
+int launch_rows(const RowK& k, size_t smem, bool pdl, cudaStream_t s) {
+  auto kern = k_sep_rows<T, L1, MODE, FWD>;
+  int per_sm = 1;
+  static SepKernelCache cache;
+  const int threads = 32 * ((std::min(k.seqs, k.n * k.rp) + 1) / 2);
+  JUBIK_TRY(cache.prepare((const void*)kern, threads, smem, &per_sm));
+  // as many CTAs as fit at once, looping over the items: the tables are built once per
+  // CTA, and the likelihood has one partial sum per CTA
+  const int64_t grid = std::min<int64_t>(
+      k.items, std::min<int64_t>(kSepMaxBlocks, (int64_t)sm_count() * per_sm));
+  return sep_launch(kern, dim3((unsigned)grid), threads, smem, pdl, s, "k_sep_rows", k);
+}
+
+template <typename T, int L1>
+int dispatch_rows(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaStream_t s) {
+  RowK k{};
+  k.a = a;
+  k.mode = mode;
+  k.nx = g.nx;
+  k.ny = g.ny;
+  k.n = g.n;
+  k.dx = g.dx;
+  k.half = g.half;
+  k.margin = g.margin;
+  k.sr_max = g.sr_max;
+  k.sc_max = g.sc_max;
+  k.K = g.K;
+  k.scale32 = (float)a.scale;
+  k.scale64 = a.scale;
+  const bool grad = mode == SEP_GRAD;
+  k.nslab = g.n / a.slab_run;
+  k.step = g.dx * a.slab_run;
+  k.height = grad ? g.K : (a.slab_run - 1) * g.dx + g.P;
+  // row pairs per item: as many as fill the sequences of one pass
+  k.seqs = row_seqs<T, L1>(g);
+  if (k.seqs < 2) {
+    set_error("separable rows: %d columns exceed the shared memory", g.ny);
+    return JUBIK_ERR_UNSUPPORTED;
+  }
+  k.rp = row_pairs(g.n, g.nx, k.seqs);
+  const int pairs = (g.nx + 1) / 2;
+  k.per = (pairs + k.rp - 1) / k.rp;
+  const int64_t items = (int64_t)a.planes * k.per;
+  if (items > 0x7fffffffLL) {
+    set_error("separable rows: too many image rows for one launch");
+    return JUBIK_ERR_UNSUPPORTED;
+  }
+  k.items = (int)items;
+  k.late = a.slab_run == 1 ? std::max(0, (g.n - 1) * g.dx - g.sr_max) : 0;
+  k.few = g.n <= k.seqs && (grad ? g.K : g.P) <= 4 * g.dx && (g.n - 1) * g.dx <= g.sc_max;
+  const int64_t reach = sep_reach(g) + k.step;
+  k.mul_dx = mulhi_divisor(g.dx, reach);
+  k.mul_step = mulhi_divisor(k.step, reach);
+  k.div_per = mulhi_divisor(k.per, items + 1);
+  const size_t smem = row_smem<T, L1>(g.n, g.ny, k.rp, k.seqs);
+  switch (mode) {
+    case SEP_SKY: return launch_rows<T, L1, SEP_SKY, true>(k, smem, pdl, s);
+    case SEP_COT:
+    case SEP_COT_READOUT: return launch_rows<T, L1, SEP_COT, true>(k, smem, pdl, s);
+    case SEP_LIKE:
+      return a.rows ? launch_rows<T, L1, SEP_LIKE, true>(k, smem, pdl, s)
+                    : launch_rows<T, L1, SEP_LIKE, false>(k, smem, pdl, s);
+    case SEP_METRIC: return launch_rows<T, L1, SEP_METRIC, true>(k, smem, pdl, s);
+    case SEP_GRAD: return launch_rows<T, L1, SEP_GRAD, false>(k, smem, pdl, s);
+    default: return launch_rows<T, L1, SEP_IMAGE, false>(k, smem, pdl, s);
+  }
+}
+
+}  // namespace
+
+template <typename T>
+int sep_rows_t(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaStream_t s) {
+  switch (g.P) {
+    case 160: return dispatch_rows<T, 10>(g, mode, a, pdl, s);
+    case 192: return dispatch_rows<T, 12>(g, mode, a, pdl, s);
+    case 256: return dispatch_rows<T, 16>(g, mode, a, pdl, s);
+    case 320: return dispatch_rows<T, 20>(g, mode, a, pdl, s);
+    case 384: return dispatch_rows<T, 24>(g, mode, a, pdl, s);
+    case 512: return dispatch_rows<T, 32>(g, mode, a, pdl, s);
+    default: break;
+  }
+  set_error("separable rows do not cover P=%d", g.P);
+  return JUBIK_ERR_UNSUPPORTED;
+}
+
+template <typename T>
+bool sep_rows_fit(const Geom& g) {
+  // (offsets within a patch column's slabs are 32-bit, divisions multiply-high)
+  if (g.dx < 2 || sep_reach(g) * (int64_t)g.nx >= (int64_t(1) << 32) ||
+      (int64_t)g.n * g.P * g.P / 2 > 0x7fffffffLL)
+    return false;
+  switch (g.P) {
+    case 160: return row_seqs<T, 10>(g) > 0;
+    case 192: return row_seqs<T, 12>(g) > 0;
+    case 256: return row_seqs<T, 16>(g) > 0;
+    case 320: return row_seqs<T, 20>(g) > 0;
+    case 384: return row_seqs<T, 24>(g) > 0;
+    case 512: return row_seqs<T, 32>(g) > 0;
+    default: return false;
+  }
+}
+
+}  // namespace jubik
