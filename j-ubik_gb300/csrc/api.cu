@@ -551,6 +551,17 @@ int finish_words(jubik_plan* p, void* hi, const void* lo, int64_t n, cudaStream_
                                : combine_words<double>(hi, lo, n, p->pdl, s);
 }
 
+// Run length is a setting of this plan (module-shared FP32 kernels at FFT side 192).
+bool sets_forward_run(const jubik_plan* p) {
+  return p->path == JUBIK_PATH_FUSED && p->spec && p->dtype == JUBIK_F32 && p->g.P == 192;
+}
+// Patches per run of the forward's columns: the setting, or the library's choice.
+int forward_run_of(const jubik_plan* p) {
+  if (!p->sep) return 1;
+  if (sets_forward_run(p) && p->fwd_run) return p->fwd_run;
+  return sep_auto_run(p->g, p->dtype);
+}
+
 // Forward of the separable path: sky rows, columns, image rows handed to `mode`
 // (onward: and on to the row spectra of the rows the adjoint starts from).
 int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMode mode, void* out,
@@ -563,9 +574,7 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
   c.tw = p->tw;
   c.wt = p->wt;
   c.slab = p->fwd_slabs;
-  // (runs exist on module-shared plans, which hold the sky spectra)
-  const int run = p->spec ? fused_fwd_run_len(g, p->dtype, p->fwd_run) : 1;
-  if (run > 1 && sep_run_fits(g, p->dtype, run)) c.run = run;
+  c.run = forward_run_of(p);
   {
     Phase ph(p, 4, s);
     SepRows r;
@@ -600,9 +609,7 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
   r.energy = energy;
   r.scale = scale;
   r.planes = g.M * g.E;
-  // after the run kernel the rows are launched in full: their looping grid, placed
-  // early between its last long CTAs, took 570 us instead of 334 us (1024^2 x 7 x 3)
-  return sep_rows(g, p->dtype, mode, r, p->pdl && c.run == 1, s);
+  return sep_rows(g, p->dtype, mode, r, p->pdl, s);
 }
 
 // Adjoint of the separable path from the row spectra in img_rows.
@@ -897,8 +904,7 @@ int jubik_plan_set_forward_run(jubik_plan* p, int32_t run_len) {
     set_error("set_forward_run: run length %d is not 0, 1, 2 or 4", run_len);
     return JUBIK_ERR_INVALID_ARGUMENT;
   }
-  if (run_len > 1 && (p->path != JUBIK_PATH_FUSED || !p->spec ||
-                      fused_fwd_run_len(p->g, p->dtype, run_len) < 0)) {
+  if (run_len > 1 && !(sets_forward_run(p) && sep_run_fits(p->g, p->dtype, run_len))) {
     set_error("set_forward_run: runs of %d patches need the module-shared FP32 kernels at FFT "
               "side 192 with 64-pixel strides, a 32-pixel margin and %d | n", run_len, run_len);
     return JUBIK_ERR_UNSUPPORTED;
@@ -913,8 +919,7 @@ int jubik_plan_forward_run(const jubik_plan* p, int32_t* run_len) {
     set_error("forward_run: null output");
     return JUBIK_ERR_INVALID_ARGUMENT;
   }
-  *run_len = (p->path == JUBIK_PATH_FUSED && p->spec)
-                 ? fused_fwd_run_len(p->g, p->dtype, p->fwd_run) : 1;
+  *run_len = sets_forward_run(p) ? forward_run_of(p) : 1;
   return JUBIK_OK;
 }
 

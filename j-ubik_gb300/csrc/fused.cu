@@ -1808,36 +1808,6 @@ int launch_pdl(KernelT kern, int64_t grid, bool pdl, cudaStream_t s, ArgsT... ar
   return cuda_status(cudaLaunchKernelEx(&cfg, kern, args...), "fused kernel launch");
 }
 
-// Geometries whose forward may run over vertically adjacent patches (sep_cols.cuh):
-// P = 192 from 64-row strides and a 32-pixel margin, a field of whole strides (no
-// clamped start), and runs of run_len (2 or 4) patch rows.
-inline bool run_geometry(const Geom& g, int run_len) {
-  return (run_len == 2 || run_len == 4) && g.P == 192 && g.dx == 64 && g.margin == 32 &&
-         g.nx == g.n * 64 && g.ny == g.n * 64 && g.n % run_len == 0 && g.M >= 2;
-}
-
-// Run length of the module-shared forward when the plan leaves it to the
-// library: runs write fewer rows (6 strides per run of 4 patches, 12 without)
-// but make fewer work items, so longer runs are taken where the busiest of the SMs
-// still does the least work at 0.87 (runs of 4) or 0.93 (runs of 2) of a unit's cost.
-inline int auto_run_len(const Geom& g) {
-  const int64_t G = sm_count(), U = g.units();
-  int best = 1;
-  double best_cost = (double)((U + G - 1) / G);
-  const int cand[2] = {2, 4};
-  const double f[2] = {0.93, 0.87};
-  for (int i = 0; i < 2; ++i) {
-    if (!run_geometry(g, cand[i])) continue;
-    const int64_t items = U / cand[i];
-    const double cost = (double)((items + G - 1) / G) * cand[i] * f[i];
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = cand[i];
-    }
-  }
-  return best;
-}
-
 // Grid of the ordered adjoint over g's units (its CTAs' unit ranges and spill
 // slots depend on it).
 template <typename T, int P>
@@ -2091,16 +2061,6 @@ int64_t fused_adj_grid(const Geom& g, int dtype) {
   if ((dtype == JUBIK_F32 ? ensure_attrs_dispatch<float>(g.P) : ensure_attrs_dispatch<double>(g.P)))
     return 0;
   return dtype == JUBIK_F32 ? ord_grid_dispatch<float>(g) : ord_grid_dispatch<double>(g);
-}
-
-// Run length the module-shared forward of geometry g uses for a request
-// (0: the library's choice): 2 or 4 for the run-ordered kernel, 1 for one
-// unit at a time.  Returns -1 for a request the geometry cannot take.
-int fused_fwd_run_len(const Geom& g, int dtype, int requested) {
-  const bool fits = dtype == JUBIK_F32 && g.P == 192;
-  if (requested == 0) return fits ? auto_run_len(g) : 1;
-  if (requested == 1) return 1;
-  return fits && run_geometry(g, requested) ? requested : -1;
 }
 
 // CTAs of the ordered adjoint over a list of problems at FFT side P that the

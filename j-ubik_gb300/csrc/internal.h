@@ -127,9 +127,6 @@ struct FusedLaunch {
 // CTAs of the ordered module-shared adjoint for geometry g (0 where the fused
 // path does not cover g.P): the count of its unit ranges and spill slots.
 int64_t fused_adj_grid(const Geom& g, int dtype);
-// Run length of the module-shared forward for a request (0 = the library's
-// choice): 1, 2 or 4, or -1 where geometry g cannot take the request.
-int fused_fwd_run_len(const Geom& g, int dtype, int requested);
 // CTAs of the ordered module-shared adjoint at FFT side P that fit on the GPU
 // at once (0 where the fused path does not cover P).
 int64_t fused_ord_capacity(int P, int dtype);

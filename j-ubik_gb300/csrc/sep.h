@@ -96,8 +96,11 @@ bool sep_rows_fit(const Geom& g);
 template <typename T>
 int sep_cols_t(const Geom& g, SepColsKind kind, const SepCols& a, bool pdl, cudaStream_t s);
 
-// Whether forward slabs of `run` patches exist: FP32, P = 192 or 384 from strides of
-// P / 3 rows, a field of whole strides, runs that tile the patch columns.
+// Whether forward slabs of `run` (2 or 4) patches exist: FP32, P = 192 or 384 from strides
+// of P / 3 rows and margins of P / 6, a field of whole strides, runs that tile the columns.
 bool sep_run_fits(const Geom& g, int dtype, int run);
+// The run length the library takes.
+int sep_auto_run(const Geom& g, int dtype);
+double sep_run_waves(const Geom& g, int run);  // waves of CTAs (sep_run_fits geometries)
 
 }  // namespace jubik

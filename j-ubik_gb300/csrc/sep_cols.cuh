@@ -19,6 +19,11 @@
 // with instruction issue; what is summed over modules or over patches therefore
 // waits in tensor memory (TMEM, 128 lanes x 512 columns per SM, otherwise unused),
 // which costs neither registers nor LSU cycles.
+//
+// The next kernel is let in at the end of a CTA's work, not at its start: row CTAs
+// that enter beside running column CTAs find the shared memory fragmented, so that
+// some SMs took two of them and others five (three fit), and the last of the looping
+// CTAs started when the first ended: 1173 us for a pass at 1024^2 x 7 x 3 against 923.
 #include "sep_dev.cuh"
 
 namespace jubik {
@@ -302,7 +307,6 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
   const cx<T>* hm = (const cx<T>*)k.a.hmain + (16 * it) * H + col;
   auto unit = [&](int m, int s) { return ((int64_t)m * k.n2 + kp0 + s) * k.E + e; };
   const int64_t hstep = (int64_t)k.n2 * k.E * (P * H);  // from module to module
-  sep_trigger();
   load_class_twiddles<T, L1>(stw, k.a.tw, NT);
   uint32_t tm = 0;
   if (D > 0) tm = col_tmem_alloc(&s_tmem, run_tmem_cols<L1, D>(k.mc));
@@ -358,6 +362,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
         }
         spectrum_to_tile<T, L1>(buf + mine, mytw, v);
       }
+      if (m + 1 == m1 && s + 1 == R) sep_trigger();
       __syncthreads();
       if (tail) {
         cx<T> v[L1];
@@ -455,7 +460,6 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
   const int64_t hstep = (int64_t)k.n2 * k.E * (P * H);
   const cx<T>* src = (const cx<T>*)k.a.rows + ((int64_t)(e * k.n + j) * k.nx) * H + cg * CG;
   const int64_t rstep = (int64_t)k.E * k.n * k.nx * H;
-  sep_trigger();
   load_class_twiddles<T, L1>(stw, k.a.tw, NT);
   cx<T> hv[16];
   if (mid) load_class<T, L1>(hb, hv);
@@ -506,6 +510,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
       }
     }
   }
+  sep_trigger();
   cx<T>* buf = tile + ((k.M & 1) ? C::TILE : 0);
   if (mid) spectrum_to_tile<T, L1>(buf + mine, mytw, acc);
   __syncthreads();
@@ -533,6 +538,22 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
 template <typename T, int L1>
 constexpr int run_shift() {
   return sizeof(T) == 4 && (L1 == 12 || L1 == 24) ? L1 / 3 : 0;
+}
+
+// Modules per CTA of the run kernel: as many as the TMEM columns of the CTAs that share
+// an SM hold.
+template <int L1, int D>
+int run_modules(int M, int per_sm) {
+  return std::min(M, std::max(1, 512 / per_sm / (2 * (L1 - D))));
+}
+
+// Waves of CTAs of the run kernel for runs of r patches.
+template <typename T, int L1>
+double run_waves(const Geom& g, int r) {
+  const int per_sm = col_ctas<T, L1>(ColT<T, L1>::SMEM, 128);
+  const int mc = run_modules<L1, run_shift<T, L1>()>(g.M, per_sm);
+  const double ctas = (double)g.E * g.n * (g.n / r) * ColT<T, L1>::NG * ((g.M + mc - 1) / mc);
+  return ctas / ((double)sm_count() * per_sm);
 }
 
 template <typename T, int L1>
@@ -575,9 +596,7 @@ int dispatch_cols(const Geom& g, SepColsKind kind, const SepCols& a, bool pdl, c
       static SepKernelCache cache;
       auto kern = k_sep_cols_fwd<T, L1, D>;
       JUBIK_TRY(cache.prepare((const void*)kern, C::NT, C::SMEM, &per_sm));
-      // as many modules per CTA as the TMEM columns of the CTAs that share an SM hold
-      k.mc = std::max(1, 512 / per_sm / (2 * (L1 - D)));
-      k.mc = std::min(k.mc, g.M);
+      k.mc = run_modules<L1, D>(g.M, per_sm);
       gd.y = (unsigned)((g.M + k.mc - 1) / k.mc);
       return sep_launch(kern, gd, C::NT, C::SMEM, pdl, s, "k_sep_cols_fwd (runs)", k);
     }

@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
   const int off = GRAD ? k.margin : 0;
   const int base_c = -k.half - k.margin + off;
   const int wx = GRAD ? k.K : P;  // window columns the overlap-add takes
-  sep_trigger();
   {
     const cx<T>* tw = (const cx<T>*)a.tw;
     for (int i = tid; i < 16 * L1; i += NT) {
@@ -413,6 +412,8 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
       }
       __syncthreads();
     }
+    // the next kernel enters beside the last item only (see sep_cols.cuh)
+    if (item + (int)gridDim.x >= k.items) sep_trigger();
     if (FWD) {
       // ---- image rows -> row spectra of every window
       for (int ch = 0; ch < nchunk; ++ch) {

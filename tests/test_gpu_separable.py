@@ -102,3 +102,40 @@ def test_cases_are_well_formed(name):
     *_, sky, _, _, R, _ = _case(name)
     lam = np.concatenate(R(sky))
     assert np.all(np.isfinite(lam)) and np.all(lam > 0)
+
+
+# (field side, patches per axis, margin, modules, energies): the library takes runs of
+# 2 (P = 192, one module), 4 (P = 384, 1 and 3 modules) and no runs (odd n)
+RUNS = [(1024, 16, 32, 1, 1), (1024, 8, 64, 1, 3), (1024, 8, 64, 3, 2), (448, 7, 32, 3, 2)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("geom", RUNS, ids=lambda g: "x".join(map(str, g)))
+def test_runs_of_the_library_match_float64(cuda, geom):
+    """FP32 plans whose run length the library chooses, against a float64 plan."""
+    nx, n, margin, M, E = geom
+    rng = np.random.default_rng(nx + M)
+    K = 2 * (nx // n)
+    u = np.arange(K) - K // 2
+    sig = rng.uniform(1.0, 5.0, size=(M, n * n, E, 1, 1))
+    psf = np.exp(-0.5 * ((u[:, None] - 0.3) ** 2 + u[None, :] ** 2) / sig ** 2) + 1e-4
+    sky = np.exp(rng.normal(size=(E, nx, nx)))
+    data = rng.poisson(3.0, size=M * E * nx * nx).astype(np.int32)
+    out = {}
+    for dtype in (F64, F32):
+        plan = ju.ResponsePlan(M, E, (nx, nx), n, margin, dtype=dtype)
+        try:
+            plan.set_psf(psf).set_data(data)
+            lam = plan.response(sky)
+            e, g = plan.energy_and_grad(sky)
+            e2, g2 = plan.energy_and_grad(sky)
+            assert float(e2) == float(e) and torch.equal(g2, g)
+            out[dtype] = lam.double().cpu().numpy(), float(e), plan.metric(None, sky)
+            out[dtype] += (plan.response_vjp(data / out[dtype][0].ravel()), g)
+        finally:
+            plan.close()
+    (l64, e64, m64, c64, g64), (l32, e32, m32, _, g32) = out[F64], out[F32]
+    assert _rel(l32, l64) < 1e-6
+    assert abs(e32 - e64) <= 1e-6 * abs(e64)
+    assert _rel(m32, m64.double().cpu().numpy()) < 1e-5
+    assert float((g32.double() - g64).norm()) < 3e-6 * float(c64.norm())
