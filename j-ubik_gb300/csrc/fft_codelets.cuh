@@ -17,18 +17,19 @@ template <bool INV, typename T> struct Dft<1, INV, T> {
 template <bool INV, typename T> struct Dft<2, INV, T> {
   __device__ __forceinline__ static void run(cx<T>* v) {
     cx<T> a = v[0];
-    v[0] = cadd<T>(a, v[1]);
-    v[1] = csub<T>(a, v[1]);
+    v[0] = padd(a, v[1]);
+    v[1] = psub(a, v[1]);
   }
 };
 
 template <bool INV, typename T> struct Dft<3, INV, T> {
   __device__ __forceinline__ static void run(cx<T>* v) {
     constexpr T s3 = (T)0.8660254037844386467637232;  // sin(2 pi / 3)
-    cx<T> t1 = cadd<T>(v[1], v[2]);
-    cx<T> t2 = mkc<T>(v[0].x - (T)0.5 * t1.x, v[0].y - (T)0.5 * t1.y);
-    cx<T> t3 = mkc<T>(s3 * (v[1].x - v[2].x), s3 * (v[1].y - v[2].y));
-    v[0] = cadd<T>(v[0], t1);
+    cx<T> t1 = padd(v[1], v[2]);
+    cx<T> t2 = pfma(both<T>((T)-0.5), t1, v[0]);
+    cx<T> d = psub(v[1], v[2]);
+    cx<T> t3 = mkc<T>(s3 * d.x, s3 * d.y);
+    v[0] = padd(v[0], t1);
     if (INV) {
       v[1] = cadd<T>(t2, cmul_i<T>(t3));
       v[2] = csub<T>(t2, cmul_i<T>(t3));
@@ -41,12 +42,12 @@ template <bool INV, typename T> struct Dft<3, INV, T> {
 
 template <bool INV, typename T> struct Dft<4, INV, T> {
   __device__ __forceinline__ static void run(cx<T>* v) {
-    cx<T> t0 = cadd<T>(v[0], v[2]);
-    cx<T> t1 = csub<T>(v[0], v[2]);
-    cx<T> t2 = cadd<T>(v[1], v[3]);
-    cx<T> t3 = csub<T>(v[1], v[3]);
-    v[0] = cadd<T>(t0, t2);
-    v[2] = csub<T>(t0, t2);
+    cx<T> t0 = padd(v[0], v[2]);
+    cx<T> t1 = psub(v[0], v[2]);
+    cx<T> t2 = padd(v[1], v[3]);
+    cx<T> t3 = psub(v[1], v[3]);
+    v[0] = padd(t0, t2);
+    v[2] = psub(t0, t2);
     if (INV) {
       v[1] = cadd<T>(t1, cmul_i<T>(t3));
       v[3] = csub<T>(t1, cmul_i<T>(t3));
@@ -67,13 +68,13 @@ template <bool INV, typename T> struct Dft<5, INV, T> {
     constexpr T c2 = (T)-0.8090169943749474241022934;  // cos(4 pi / 5)
     constexpr T s1 = (T)0.9510565162951535721164393;   // sin(2 pi / 5)
     constexpr T s2 = (T)0.5877852522924731291687060;   // sin(4 pi / 5)
-    const cx<T> t1 = cadd<T>(v[1], v[4]), t2 = cadd<T>(v[2], v[3]);
-    const cx<T> t3 = csub<T>(v[1], v[4]), t4 = csub<T>(v[2], v[3]);
-    const cx<T> a1 = mkc<T>(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    const cx<T> a2 = mkc<T>(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
+    const cx<T> t1 = padd(v[1], v[4]), t2 = padd(v[2], v[3]);
+    const cx<T> t3 = psub(v[1], v[4]), t4 = psub(v[2], v[3]);
+    const cx<T> a1 = pfma(both<T>(c2), t2, pfma(both<T>(c1), t1, v[0]));
+    const cx<T> a2 = pfma(both<T>(c1), t2, pfma(both<T>(c2), t1, v[0]));
     const cx<T> b1 = mkc<T>(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
     const cx<T> b2 = mkc<T>(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
-    v[0] = cadd<T>(v[0], cadd<T>(t1, t2));
+    v[0] = padd(v[0], padd(t1, t2));
     if (INV) {
       v[1] = cadd<T>(a1, cmul_i<T>(b1));
       v[4] = csub<T>(a1, cmul_i<T>(b1));

@@ -91,6 +91,31 @@ __device__ __forceinline__ void two_quotients(double a, double b, double x, doub
   qb = b / x;
 }
 
+// The same for two pairs of quotients.
+__device__ __forceinline__ void two_quotients(float2 a, float2 b, float2 x, float2& qa,
+                                              float2& qb) {
+  const bool plain = fabsf(x.x) > 1e-18f && fabsf(x.x) < 1e18f && fabsf(a.x) < 1e18f &&
+                     fabsf(x.y) > 1e-18f && fabsf(x.y) < 1e18f && fabsf(a.y) < 1e18f;
+  if (!plain) {
+    two_quotients(a.x, b.x, x.x, qa.x, qb.x);
+    two_quotients(a.y, b.y, x.y, qa.y, qb.y);
+    return;
+  }
+  float2 r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+  const float2 m = make_float2(-x.x, -x.y);
+  qa = pmul(a, r);
+  qb = pmul(b, r);
+  qa = pfma(pfma(m, qa, a), r, qa);
+  qb = pfma(pfma(m, qb, b), r, qb);
+}
+__device__ __forceinline__ void two_quotients(double2 a, double2 b, double2 x, double2& qa,
+                                              double2& qb) {
+  two_quotients(a.x, b.x, x.x, qa.x, qb.x);
+  two_quotients(a.y, b.y, x.y, qa.y, qb.y);
+}
+
 // One pixel: lam = eps * conv where a pixel is read out (count >= 0), the
 // energy terms, the residual eps * (1 - d/lam) (0 elsewhere) and the metric
 // weight eps^2 / lam (0 elsewhere) that later Fisher-metric products apply to
@@ -111,6 +136,42 @@ __device__ __forceinline__ void poisson_px(T conv, T ep, int32_t d, T& w_o, T& r
   T q;
   two_quotients(ep * ep, dd, lam, w_o, q);
   res_o = ep * ((T)1 - q);
+}
+
+// Compensated sums of two sequences of values, or of products (fused with the
+// compensation's subtraction): nc is minus Kahan's c.
+template <typename T>
+struct Kahan2 {
+  cx<T> s = mkc<T>((T)0, (T)0), nc = mkc<T>((T)0, (T)0);
+  __device__ __forceinline__ void add_y(cx<T> y) {
+    const cx<T> t = padd(s, y);
+    nc = psub(y, psub(t, s));
+    s = t;
+  }
+  __device__ __forceinline__ void add(cx<T> v) { add_y(padd(v, nc)); }
+  __device__ __forceinline__ void add_product(cx<T> a, cx<T> b) { add_y(pfma(a, b, nc)); }
+  __device__ __forceinline__ double value() const {
+    return ((double)s.x + (double)nc.x) + ((double)s.y + (double)nc.y);
+  }
+};
+
+// Two pixels (of two image rows) at once, as poisson_px.
+template <typename T>
+__device__ __forceinline__ void poisson_px2(cx<T> conv, cx<T> ep, const int32_t (&d)[2],
+                                            cx<T>& w_o, cx<T>& res_o, Kahan2<T>& s_lam,
+                                            Kahan2<T>& s_dlog) {
+  const bool a = d[0] >= 0, b = d[1] >= 0;
+  const cx<T> lam = pmul(ep, conv);
+  // pixels that are not read out: lam = 1 and a count of 0 enter nowhere
+  const cx<T> x = mkc<T>(a ? lam.x : (T)1, b ? lam.y : (T)1);
+  const cx<T> dd = mkc<T>(a ? (T)d[0] : (T)0, b ? (T)d[1] : (T)0);
+  s_lam.add(mkc<T>(a ? lam.x : (T)0, b ? lam.y : (T)0));
+  s_dlog.add_product(dd, mkc<T>(log(x.x), log(x.y)));
+  cx<T> w, q;
+  two_quotients(pmul(ep, ep), dd, x, w, q);
+  const cx<T> res = pmul(ep, psub(both<T>((T)1), q));
+  w_o = mkc<T>(a ? w.x : (T)0, b ? w.y : (T)0);
+  res_o = mkc<T>(a ? res.x : (T)0, b ? res.y : (T)0);
 }
 
 }  // namespace jubik

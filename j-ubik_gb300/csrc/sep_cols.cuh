@@ -199,16 +199,16 @@ __device__ __forceinline__ void load_sky_rows(const ColK& k, const cx<T>* src,
                                               int rb, int n2, cx<T> (&v)[L1]) {
   constexpr int H = 8 * L1;
   const T* __restrict__ wt = (const T*)k.a.wt;
+  T w[L1];  // (every load is issued before the first product)
 #pragma unroll
   for (int i = 0; i < L1; ++i) {
     const int y = n2 + 16 * i, ya = y - k.margin, row = rb + y;
-    v[i] = mkc<T>((T)0, (T)0);
-    if (ya >= 0 && ya < k.K && row >= 0 && row < k.nx) {
-      const cx<T> z = src[(int64_t)row * H];
-      const T w = wt[ya];
-      v[i] = mkc<T>(w * z.x, w * z.y);
-    }
+    const bool ok = (unsigned)ya < (unsigned)k.K && (unsigned)row < (unsigned)k.nx;
+    v[i] = ok ? src[(int64_t)row * H] : mkc<T>((T)0, (T)0);
+    w[i] = ok ? wt[ya] : (T)0;
   }
+#pragma unroll
+  for (int i = 0; i < L1; ++i) v[i] = mkc<T>(w[i] * v[i].x, w[i] * v[i].y);
 }
 
 // the 16 values of a class: rows 16 cls + q of the (P, H) array h, column col

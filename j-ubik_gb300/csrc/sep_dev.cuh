@@ -25,15 +25,16 @@ __device__ __forceinline__ int sep_div(int u, int d, uint32_t mul) {
   return mul ? (int)__umulhi((uint32_t)u, mul) : u / d;
 }
 
-// (a + conj(b)) / 2 and (a - conj(b)) / (2i): the spectra of the two real rows
-// of a pair from the pair's transform at k and -k; and their inverses
+// a + conj(b) and (a - conj(b)) / i: twice the spectra of the two real rows of a
+// pair from the pair's transform at k and -k (the rows are halved before); and
+// their inverses
 template <typename T>
 __device__ __forceinline__ cx<T> split_a(cx<T> a, cx<T> b) {
-  return mkc<T>((T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y));
+  return mkc<T>(a.x + b.x, a.y - b.y);
 }
 template <typename T>
 __device__ __forceinline__ cx<T> split_b(cx<T> a, cx<T> b) {
-  return mkc<T>((T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x));
+  return mkc<T>(a.y + b.y, b.x - a.x);
 }
 template <typename T>
 __device__ __forceinline__ cx<T> join_p(cx<T> a, cx<T> b) {  // a + i b

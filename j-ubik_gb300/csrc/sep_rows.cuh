@@ -98,6 +98,53 @@ __device__ __forceinline__ void row_twiddles(const double2* tw, int q, double2& 
   b = tw[q + 1];
 }
 
+// Joins the two rows' values of kx = lane + 32 t and writes those of the pair's sequence
+// at kx and P - kx (kx = 0: the packed real kx = 0 and kx = P / 2 values).
+template <typename T, int L1>
+__device__ __forceinline__ void row_join(const cx<T> (&v)[2], int t, cx<T>* wp, cx<T>* wm,
+                                         int lane) {
+  const bool dc = t == 0 && lane == 0;
+  wp[34 * t] = dc ? mkc<T>(v[0].x, v[1].x) : join_p<T>(v[0], v[1]);
+  (dc ? wp + row_slot(8 * L1) : wm - 34 * t)[0] =
+      dc ? mkc<T>(v[0].y, v[1].y) : join_m<T>(v[0], v[1]);
+}
+
+// Spectra of a row pair in one window: the sum of up to N slabs, in order.  The loads of
+// three steps are issued before the first sum: with one loop for up to three slabs the
+// compiler interleaved loads and sums, and the likelihood's rows took 331 us at
+// 1024^2 x 7 x 3 and 381 at side 384, now 272 and 268 (2.8 -> 3.4 TB/s).
+template <typename T, int L1, int N>
+__device__ __forceinline__ void row_load(const cx<T>* p, const int (&o)[2][3], const int (&m)[2],
+                                         cx<T>* wp, cx<T>* wm, int lane) {
+  constexpr int H = 8 * L1, STEPS = (H + 31) / 32, G = sizeof(T) == 4 ? 3 : 1;
+#pragma unroll
+  for (int t0 = 0; t0 < STEPS; t0 += G) {
+    cx<T> z[G][2][N];
+#pragma unroll
+    for (int t = t0; t < t0 + G && t < STEPS; ++t) {
+      const bool in = H % 32 == 0 || lane + 32 * t < H;
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+          z[t - t0][b][u] =
+              in && u < m[b] ? p[o[b][u] + 32 * t] : mkc<T>((T)0, (T)0);
+    }
+#pragma unroll
+    for (int t = t0; t < t0 + G && t < STEPS; ++t) {
+      if (H % 32 && lane + 32 * t >= H) break;
+      cx<T> v[2];
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        v[b] = z[t - t0][b][0];
+#pragma unroll
+        for (int u = 1; u < N; ++u) v[b] = cadd<T>(v[b], z[t - t0][b][u]);
+      }
+      row_join<T, L1>(v, t, wp, wm, lane);
+    }
+  }
+}
+
 // DFT-L1 of class `ca` of a sequence, in place
 template <typename T, int L1, bool INV>
 __device__ __forceinline__ void row_dft_l1(cx<T>* seq, int ca) {
@@ -167,7 +214,7 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
   __syncthreads();
   const cx<T>* mytw = stw + kRowTw * cls;
   const T scale = row_scale<T>(k);
-  Kahan<T> s_lam, s_dlog;
+  Kahan2<T> s_lam, s_dlog;
   const int nchunk = (n * k.rp + k.seqs - 1) / k.seqs;  // > 1 only when rp == 1
 
   for (int item = blockIdx.x; item < k.items; item += gridDim.x) {
@@ -205,32 +252,30 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
           const cx<T>* p = (const cx<T>*)a.slab + ((int64_t)pl * n + j) * hs * k.nslab + lane;
           cx<T>* wp = buf + s * WP + slot_p;
           cx<T>* wm = buf + s * WP + slot_m;
+          const int most = max(m[0], m[1]);
+          if (most <= 1) {
+            row_load<T, L1, 1>(p, o, m, wp, wm, lane);
+          } else if (most == 2) {
+            row_load<T, L1, 2>(p, o, m, wp, wm, lane);
+          } else if (most == 3) {
+            row_load<T, L1, 3>(p, o, m, wp, wm, lane);
+          } else {  // margins beyond half a stride: more slabs
+            const int late = k.late * H;
+#pragma unroll 1
+            for (int t = 0; t < (H + 31) / 32; ++t) {
+              if (H % 32 && lane + 32 * t >= H) break;
+              cx<T> v[2];
 #pragma unroll
-          for (int t = 0; t < (H + 31) / 32; ++t) {
-            if (H % 32 && lane + 32 * t >= H) break;
-            cx<T> v[2];
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              const cx<T> z = mkc<T>((T)0, (T)0);
-              const cx<T> v0 = 0 < m[b] ? p[o[b][0] + 32 * t] : z;
-              const cx<T> v1 = 1 < m[b] ? p[o[b][1] + 32 * t] : z;
-              const cx<T> v2 = 2 < m[b] ? p[o[b][2] + 32 * t] : z;
-              v[b] = cadd<T>(cadd<T>(v0, v1), v2);
+              for (int b = 0; b < 2; ++b) {
+                v[b] = mkc<T>((T)0, (T)0);
+                const int step = hs - k.step * H, first = o[b][0];
+#pragma unroll 4
+                for (int u = 0; u < m[b]; ++u)
+                  v[b] = cadd<T>(v[b], p[first + u * step + 32 * t +
+                                         (u && lo[b] + u == k.nslab - 1 ? late : 0)]);
+              }
+              row_join<T, L1>(v, t, wp, wm, lane);
             }
-            if (max(m[0], m[1]) > 3) {  // margins beyond a stride: more slabs
-#pragma unroll
-              for (int b = 0; b < 2; ++b)
-                for (int u = 3; u < m[b]; ++u) {
-                  const int i = lo[b] + u;
-                  v[b] = cadd<T>(v[b], p[i * hs + (row0 + b - base_c - i * k.step +
-                                                   (i == k.nslab - 1 ? k.late : 0)) * H + 32 * t]);
-                }
-            }
-            // join the two rows (kx = 0: the packed real kx = 0 and kx = P / 2 values)
-            const bool dc = t == 0 && lane == 0;
-            wp[34 * t] = dc ? mkc<T>(v[0].x, v[1].x) : join_p<T>(v[0], v[1]);
-            (dc ? wp + row_slot(H) : wm - 34 * t)[0] =
-                dc ? mkc<T>(v[0].y, v[1].y) : join_m<T>(v[0], v[1]);
           }
         }
         __syncwarp();
@@ -311,9 +356,9 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
                   z1 = mkc<T>(g1 * z1.x, g1 * z1.y);
                   z2 = mkc<T>(g2 * z2.x, g2 * z2.y);
                 }
-                const cx<T> t = cadd<T>(z0, z1);
-                const cx<T> y = csub<T>(z2, csub<T>(csub<T>(t, z0), z1));
-                sum = cadd<T>(t, y);
+                const cx<T> t = padd(z0, z1);
+                const cx<T> y = psub(z2, psub(psub(t, z0), z1));
+                sum = padd(t, y);
                 if (cw > 3) {
                   cx<T> z3 = w[3 * S];
                   if (GRAD) {
@@ -352,28 +397,34 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
                   continue;
                 }
               }
-              const T v[2] = {scale * sum.x, scale * sum.y};
-              T o[2] = {(T)0, (T)0};
+              const cx<T> v = pmul(both<T>(scale), sum);
+              const int64_t p = px0 + x;
+              if (MODE == SEP_LIKE) {
+                cx<T> wgt, res;
+                poisson_px2<T>(v, mkc<T>(f[u][0], f[u][1]), ix[u], wgt, res, s_lam, s_dlog);
+                __stcs((T*)a.wts + p, wgt.x);
+                if (two) __stcs((T*)a.wts + p + ny, wgt.y);
+                if (FWD) line[r * ny + x] = pmul(both<T>((T)0.5), res);
+              } else if (MODE == SEP_METRIC) {
+                if (FWD)
+                  line[r * ny + x] = mkc<T>((T)0.5 * (f[u][0] * v.x),
+                                            two ? (T)0.5 * (f[u][1] * v.y) : (T)0);
+              } else {
 #pragma unroll
-              for (int b = 0; b < 2; ++b) {
-                if (b && !two) break;
-                const int64_t p = px0 + (int64_t)b * ny + x;
-                if (MODE == SEP_LIKE) {
-                  T wgt;
-                  poisson_px<T>(v[b], f[u][b], ix[u][b], wgt, o[b], s_lam, s_dlog);
-                  __stcs((T*)a.wts + p, wgt);
-                } else if (MODE == SEP_METRIC) {
-                  o[b] = f[u][b] * v[b];
-                } else if (MODE == SEP_GRAD || k.mode == SEP_IMAGE) {
-                  ((T*)a.out)[p] = v[b];
-                } else if (k.mode == SEP_READOUT) {
-                  if (ix[u][b] >= 0) ((T*)a.out)[ix[u][b]] = eps ? f[u][b] * v[b] : v[b];
-                } else {  // SEP_WEIGHTS
-                  const T ep = f[u][b];
-                  ((T*)a.wts)[p] = ix[u][b] < 0 ? (T)0 : (ep * ep) / (ep * v[b]);
+                for (int b = 0; b < 2; ++b) {
+                  if (b && !two) break;
+                  const int64_t pb = p + (int64_t)b * ny;
+                  const T vb = b ? v.y : v.x;
+                  if (MODE == SEP_GRAD || k.mode == SEP_IMAGE) {
+                    ((T*)a.out)[pb] = vb;
+                  } else if (k.mode == SEP_READOUT) {
+                    if (ix[u][b] >= 0) ((T*)a.out)[ix[u][b]] = eps ? f[u][b] * vb : vb;
+                  } else {  // SEP_WEIGHTS
+                    const T ep = f[u][b];
+                    ((T*)a.wts)[pb] = ix[u][b] < 0 ? (T)0 : (ep * ep) / (ep * vb);
+                  }
                 }
               }
-              if (FWD) line[r * ny + x] = mkc<T>(o[0], o[1]);
             }
           }
         }
@@ -385,29 +436,56 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
         const int row0 = 2 * (t0 + r);
         if (row0 >= nx) break;
         const bool two = row0 + 1 < nx;
-#pragma unroll 2
-        for (int x = tid; x < ny; x += NT) {
-          T o[2] = {(T)0, (T)0};
+        // columns loaded together: with two loads at a time the scattered readout rows of
+        // 1024^2 x 1 x 3 took 52 us, now 27 (36 with two columns)
+        constexpr int U = 4;
+        for (int xb = tid; xb < ny; xb += U * NT) {
+          T o[U][2];
+          if (MODE == SEP_SKY || k.mode == SEP_COT) {
+            const T* in = (const T*)a.in + (MODE == SEP_SKY
+                                                ? pl * a.in_ps + (int64_t)row0 * a.in_rs
+                                                : ((int64_t)pl * nx + row0) * ny);
+            const int64_t rs = MODE == SEP_SKY ? a.in_rs : ny;
 #pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            if (b && !two) break;
-            if (MODE == SEP_SKY) {
-              const T v = ((const T*)a.in)[pl * a.in_ps + (int64_t)(row0 + b) * a.in_rs + x];
-              o[b] = a.in_exp ? exp(v) : v;
-            } else {
-              const int64_t p = ((int64_t)pl * nx + row0 + b) * ny + x;
-              if (k.mode == SEP_COT) {
-                o[b] = ((const T*)a.in)[p];
-              } else {  // SEP_COT_READOUT
-                const int32_t i = a.ridx[p];
-                if (i >= 0) {
-                  const T v = ((const T*)a.in)[i];
-                  o[b] = eps ? eps[p] * v : v;
-                }
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) {
+                const int x = xb + u * NT;
+                o[u][b] = x < ny && (b == 0 || two) ? in[b * rs + x] : (T)0;
               }
-            }
+          } else {  // SEP_COT_READOUT
+            int32_t ix[U][2];
+            T f[U][2];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) {
+                const int x = xb + u * NT;
+                const int64_t p = ((int64_t)pl * nx + row0 + b) * ny + x;
+                const bool ok = x < ny && (b == 0 || two);
+                ix[u][b] = ok ? a.ridx[p] : -1;
+                f[u][b] = ok && eps ? eps[p] : (T)1;
+              }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int b = 0; b < 2; ++b)
+                o[u][b] = ix[u][b] >= 0 ? ((const T*)a.in)[ix[u][b]] : (T)0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) o[u][b] = ix[u][b] >= 0 ? f[u][b] * o[u][b] : (T)0;
           }
-          line[r * ny + x] = mkc<T>(o[0], o[1]);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int x = xb + u * NT;
+            if (x >= ny) break;
+            if (MODE == SEP_SKY && a.in_exp) {
+              o[u][0] = exp(o[u][0]);
+              o[u][1] = two ? exp(o[u][1]) : (T)0;
+            }
+            line[r * ny + x] = pmul(both<T>((T)0.5), mkc<T>(o[u][0], o[u][1]));
+          }
         }
       }
       __syncthreads();
@@ -460,7 +538,7 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
         if (q0 + (lane >> 4) < cnt) row_dft_l1<T, L1, false>(buf + (q0 + (lane >> 4)) * WP, lane & 15);
         __syncwarp();
 #pragma unroll 1
-        for (int s = q0; s < q0 + 2 && s < cnt; ++s) {  // split into the two rows' spectra
+        for (int s = q0; s < q0 + 2 && s < cnt; ++s) {  // split the halved rows' sum
           const int r = k.rp == 1 ? 0 : s / jn, j = j0 + s - r * jn;
           const int row0 = 2 * (t0 + r);
           if (row0 >= nx) break;
@@ -473,8 +551,10 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
             if (H % 32 && lane + 32 * t >= H) break;
             const bool dc = t == 0 && lane == 0;
             const cx<T> zp = wp[34 * t], zm = (dc ? wp + row_slot(H) : wm - 34 * t)[0];
-            dst[32 * t] = dc ? mkc<T>(zp.x, zm.x) : split_a<T>(zp, zm);
-            if (two) dst[H + 32 * t] = dc ? mkc<T>(zp.y, zm.y) : split_b<T>(zp, zm);
+            dst[32 * t] = dc ? padd(mkc<T>(zp.x, zm.x), mkc<T>(zp.x, zm.x)) : split_a<T>(zp, zm);
+            if (two)
+              dst[H + 32 * t] =
+                  dc ? padd(mkc<T>(zp.y, zm.y), mkc<T>(zp.y, zm.y)) : split_b<T>(zp, zm);
           }
         }
         __syncwarp();  // this warp's sequences have been read
