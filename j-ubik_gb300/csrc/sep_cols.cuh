@@ -211,11 +211,23 @@ __device__ __forceinline__ void load_sky_rows(const ColK& k, const cx<T>* src,
   for (int i = 0; i < L1; ++i) v[i] = mkc<T>(w[i] * v[i].x, w[i] * v[i].y);
 }
 
-// the 16 values of a class: rows 16 cls + q of the (P, H) array h, column col
-template <typename T, int L1>
+__device__ __forceinline__ float2 col_load_past_l1(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];"
+               : "=f"(v.x), "=f"(v.y)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 col_load_past_l1(const double2* p) { return __ldg(p); }
+// the 16 values of a class: rows 16 cls + q of the (P, H) array h, column col.  PAST_L1:
+// lines that are read once leave the L1 to the other loads in flight.  The adjoint takes
+// it (FP32; side 384 at 1024^2 x 7 x 3: 305 -> 294 us, side 192 at one module 68.9 ->
+// 66.8); the forward, whose sky rows are re-read from L1, does not (291 -> 302).
+template <typename T, int L1, bool PAST_L1>
 __device__ __forceinline__ void load_class(const cx<T>* h, cx<T> (&v)[16]) {
 #pragma unroll
-  for (int q = 0; q < 16; ++q) v[q] = __ldg(h + q * (8 * L1));
+  for (int q = 0; q < 16; ++q)
+    v[q] = PAST_L1 ? col_load_past_l1(h + q * (8 * L1)) : __ldg(h + q * (8 * L1));
 }
 // twiddles q and q + 1 (q even) of a class in one 16-byte load (FP32)
 __device__ __forceinline__ void two_twiddles(const float2* tw, int q, float2& a, float2& b) {
@@ -313,7 +325,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
   sep_wait();
   const cx<T>* hb = hm + unit(m0, 0) * (P * H);
   cx<T> hv[16];
-  if (mid) load_class<T, L1>(hb, hv);
+  if (mid) load_class<T, L1, false>(hb, hv);
   const cx<T>* mytw = stw + C::TWP * it;
   const int mine = C::at(16 * it, c), myrow = C::at(it, c);
   const int height = D == 0 ? P : (R - 1) * k.dx + P;
@@ -349,10 +361,10 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
         for (int q = 0; q < 16; ++q) v[q] = cmul<T>(sp[q], hv[q]);
         if (m + 1 < m1) {
           hb += hstep;
-          load_class<T, L1>(hb, hv);
+          load_class<T, L1, false>(hb, hv);
         } else if (s + 1 < R) {
           hb = hm + unit(m0, s + 1) * (P * H);
-          load_class<T, L1>(hb, hv);
+          load_class<T, L1, false>(hb, hv);
         }
         if (c0) {
           const cx<T>* be = (const cx<T>*)k.a.hnyq + unit(m, s) * P + 16 * it;
@@ -462,7 +474,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
   const int64_t rstep = (int64_t)k.E * k.n * k.nx * H;
   load_class_twiddles<T, L1>(stw, k.a.tw, NT);
   cx<T> hv[16];
-  if (mid) load_class<T, L1>(hb, hv);
+  if (mid) load_class<T, L1, true>(hb, hv);
   sep_wait();
   col_fetch_rows<T, L1>(tile, src, rb, k.nx, tid);
   const cx<T>* mytw = stw + C::TWP * it;
@@ -493,7 +505,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
 #pragma unroll
       for (int q = 0; q < 16; ++q) acc[q] = cadd<T>(acc[q], cmulc<T>(v[q], hv[q]));
       hb += hstep;
-      if (m + 1 < k.M) load_class<T, L1>(hb, hv);
+      if (m + 1 < k.M) load_class<T, L1, true>(hb, hv);
       if (c0) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) w0[16 * it + q] = v[q];
