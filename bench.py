@@ -726,30 +726,29 @@ def main():
     d2h = gh[0].numel() * gh[0].element_size() + 8
 
     # roofline of the dominant kernel (algorithmic = compulsory DRAM bytes per launch)
-    U = M * E * inst.n_patches ** 2
-    NP = E * inst.n_patches ** 2
-    P = inst.P
+    n, P = inst.n_patches, inst.P
+    U = M * E * n ** 2
+    NP = E * n ** 2
+    row = P // 2 * 8                         # one row spectrum
     spec = U * (P * P // 2 + P) * 8          # PSF spectra, read once per launch
-    pspec = NP * P * (P // 2) * 8            # shared patch spectra
     img, sky = M * E * nx * nx * 4, E * nx * nx * 4
-    fft_unit = 5.0 * P * P * np.log2(P)      # one real 2-D FFT of side P (5 N log2 N / 2)
+    sky_rows, img_rows = E * n * nx * row, M * E * n * nx * row
+    r = plan.forward_run                     # patches per slab of the forward columns
+    slabs = M * E * n * (n // r) * ((r - 1) * inst.dx + P) * row
+    grad_slabs = NP * 2 * inst.dx * row
+    cols = 2.5 * P * P * np.log2(P)          # the columns of one real 2-D FFT of side P
+    rows = 2.5 * P * np.log2(P)              # one real row
     mul_unit = 6.0 * P * (P // 2)
-    shared = plan.shared_spectra
-    # whole 64-row block rows per patch output (P 192, stride 64, margin 32, runs of
-    # 4 patch rows, 2+ modules): the forward runs the run-ordered kernel
-    run = (P == 192 and inst.dx == 64 and inst.margin == 32 and nx == inst.n_patches * 64
-           and inst.n_patches % 4 == 0 and M >= 2)
-    fwd_kernel = "k_fwd_run<float,192>" if run else "k_fwd_from_spec<float,192>"
-    kinfo = {  # phase -> (kernel, bytes, flops)
-        # the forward leaves both words of the exact two-word image sum
-        "forward": (fwd_kernel if shared else "k_fused<float,192,fwd>",
-                    spec + (pspec if shared else sky) + 2 * img,
-                    U * (fft_unit * (1 if shared else 2) + mul_unit)),
-        "adjoint": ("k_adj_to_spec_ord<float,192>" if shared else "k_fused<float,192,adj>",
-                    spec + img + (pspec if shared else sky),
-                    U * (fft_unit * (1 if shared else 2) + mul_unit)),
-        "forward_patch": ("k_sky_spec<float,192>", sky + pspec, NP * fft_unit),
-        "adjoint_patch": ("k_adj_from_spec<float,192>", pspec + sky, NP * fft_unit),
+    kinfo = {  # phase -> (kernel, bytes, flops): the separable path (FFT side 192)
+        "forward_patch": ("k_sep_rows<float,12,sky>", sky + sky_rows, E * n * nx * rows),
+        "forward": ("k_sep_cols_fwd<float,12>", spec + sky_rows + slabs,
+                    (U + NP) * cols + U * mul_unit),
+        # exposure and counts in, metric weights out
+        "likelihood": ("k_sep_rows<float,12,likelihood>", slabs + 3 * img + img_rows,
+                       2 * M * E * n * nx * rows),
+        "adjoint": ("k_sep_cols_adj<float,12>", spec + img_rows + grad_slabs,
+                    (U + NP) * cols + U * mul_unit),
+        "adjoint_patch": ("k_sep_rows<float,12,gradient>", grad_slabs + sky, E * n * nx * rows),
     }
     dom = max((k for k in kinfo if per_launch.get(k, 0.0) > 0), key=lambda k: per_launch[k])
     dom_name, dom_bytes, flops = kinfo[dom]

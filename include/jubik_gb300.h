@@ -164,7 +164,10 @@ JUBIK_API int jubik_metric_apply(jubik_plan* plan, const void* x, const void* v,
  * kernel, 1 adjoint per-unit PSF kernel, 2 likelihood / readout kernels,
  * 3 memsets, 4 forward per-patch sky-spectrum kernel, 5 adjoint per-patch
  * inverse kernel (4 and 5 run when modules share patch spectra), 6 the pass
- * that adds the low words of the gradient's exact two-word sum (fused path). */
+ * that adds the low words of the gradient's exact two-word sum (fused path).
+ * Separable plans (FFT sides 160 .. 512): 4 sky rows, 0 forward columns, 2 the
+ * rows that end or turn the pass (with the likelihood), 1 adjoint columns, 5
+ * gradient rows. */
 #define JUBIK_PHASES 7
 /* Programmatic dependent launch between the kernels of one plan call (default
  * on; no counterpart in the reference): each kernel may be scheduled onto the
