@@ -68,12 +68,20 @@ __device__ __forceinline__ void block_reduce2_of(double a, double b, double* sa,
   }
 }
 
+// Whether two_quotients may form a / x: neither a quotient nor the residual a - x q leaves
+// the normal range, so the residual is exact.  (b / x of a count b needs no more: b is 0
+// or at least 1.)
+__device__ __forceinline__ bool plain_quotient(float a, float x) {
+  const float m = fabsf(x), n = fabsf(a);
+  return m > 1e-18f && m < 1e18f && (n == 0.0f || (n > 1e-18f && n < 1e18f));
+}
+
 // a / x and b / x from one reciprocal, each quotient corrected by its residual (one
-// Newton step on the quotient, Markstein 1990): within rounding of the exact
-// quotients for x of ordinary size; others divide.
+// Newton step on the quotient, Markstein 1990).  Tested for the bits of the division over
+// that range of a and x; outside it, the division.  (Two divisions a pixel in their place:
+// 272 -> 315 us for the likelihood's rows at 1024^2 x 7 x 3.)
 __device__ __forceinline__ void two_quotients(float a, float b, float x, float& qa, float& qb) {
-  const bool plain = fabsf(x) > 1e-18f && fabsf(x) < 1e18f && fabsf(a) < 1e18f;
-  if (!plain) {
+  if (!plain_quotient(a, x)) {
     qa = a / x;
     qb = b / x;
     return;
@@ -94,9 +102,7 @@ __device__ __forceinline__ void two_quotients(double a, double b, double x, doub
 // The same for two pairs of quotients.
 __device__ __forceinline__ void two_quotients(float2 a, float2 b, float2 x, float2& qa,
                                               float2& qb) {
-  const bool plain = fabsf(x.x) > 1e-18f && fabsf(x.x) < 1e18f && fabsf(a.x) < 1e18f &&
-                     fabsf(x.y) > 1e-18f && fabsf(x.y) < 1e18f && fabsf(a.y) < 1e18f;
-  if (!plain) {
+  if (!(plain_quotient(a.x, x.x) && plain_quotient(a.y, x.y))) {
     two_quotients(a.x, b.x, x.x, qa.x, qb.x);
     two_quotients(a.y, b.y, x.y, qa.y, qb.y);
     return;
