@@ -280,6 +280,9 @@ struct jubik_plan {
   // separable path (sep.h): the entry points of this plan run its row and column
   // kernels; a fused plan's other buffers then serve grouped launches only
   bool sep = false;
+  void* ramp = nullptr;  // (K) window weights times (dx - 1) / 2^ramp_log2, exact
+  int ramp_log2 = 0;
+  double* gains = nullptr;  // (2, P) gains less one of the column and row transforms (FP32)
   void* sky_rows = nullptr;
   void* fwd_slabs = nullptr;
   void* img_rows = nullptr;
@@ -557,6 +560,32 @@ int finish_words(jubik_plan* p, void* hi, const void* lo, int64_t n, cudaStream_
                                : combine_words<double>(hi, lo, n, p->pdl, s);
 }
 
+// Window weights of the separable kernels: k / 2^ramp_log2 for the bilinear k / (dx - 1),
+// exact in either precision, so that only the products with them round; sep_scale has the
+// rest of the factor.
+int upload_sep_tables(jubik_plan* p) {
+  const int dx = p->g.dx;
+  p->ramp_log2 = 0;
+  while ((1 << p->ramp_log2) < dx - 1) ++p->ramp_log2;
+  JUBIK_TRY(p->alloc(&p->ramp, p->g.K * p->esz));
+  std::vector<float> f(p->g.K);
+  std::vector<double> d(p->g.K);
+  for (int i = 0; i < p->g.K; ++i) {
+    d[i] = std::ldexp((double)std::min(i, p->g.K - 1 - i), -p->ramp_log2);
+    f[i] = (float)d[i];
+  }
+  JUBIK_TRY_CUDA(cudaMemcpy(p->ramp, p->esz == 4 ? (void*)f.data() : (void*)d.data(),
+                            p->g.K * p->esz, cudaMemcpyHostToDevice));
+  if (p->dtype != JUBIK_F32) return JUBIK_OK;
+  std::vector<double> g, gx;
+  sep_gains(p->g.P, g, gx);
+  g.insert(g.end(), gx.begin(), gx.end());
+  JUBIK_TRY(p->alloc((void**)&p->gains, g.size() * sizeof(double)));
+  return cuda_status(cudaMemcpy(p->gains, g.data(), g.size() * sizeof(double),
+                                cudaMemcpyHostToDevice),
+                     "upload gains");
+}
+
 // Run length is a setting of this plan (module-shared FP32 kernels at FFT side 192).
 bool sets_forward_run(const jubik_plan* p) {
   return p->path == JUBIK_PATH_FUSED && p->spec && p->dtype == JUBIK_F32 && p->g.P == 192;
@@ -566,6 +595,15 @@ int forward_run_of(const jubik_plan* p) {
   if (!p->sep) return 1;
   if (sets_forward_run(p) && p->fwd_run) return p->fwd_run;
   return sep_auto_run(p->g, p->dtype);
+}
+
+// The factor of a pass in two words: `scale`, and what the exact weights leave out of the
+// bilinear ones along both axes.
+void sep_scale(const jubik_plan* p, double scale, SepRows* r) {
+  const double a = std::ldexp(scale, 2 * p->ramp_log2);
+  const double d = (double)(p->g.dx - 1) * (p->g.dx - 1);
+  r->scale = a / d;
+  r->scale_lo = std::fma(-r->scale, d, a) / d;
 }
 
 // Forward of the separable path: sky rows, columns, image rows handed to `mode`
@@ -578,7 +616,7 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
   c.hmain = p->hmain;
   c.hnyq = p->hnyq;
   c.tw = p->tw;
-  c.wt = p->wt;
+  c.wt = p->ramp;
   c.slab = p->fwd_slabs;
   c.run = forward_run_of(p);
   {
@@ -590,7 +628,7 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
     r.in_exp = view.exp ? 1 : 0;
     r.rows = p->sky_rows;
     r.tw = p->tw;
-    r.wt = p->wt;
+    r.wt = p->ramp;
     r.planes = g.E;
     JUBIK_TRY(sep_rows(g, p->dtype, SEP_SKY, r, p->pdl, s));
   }
@@ -605,7 +643,7 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
   r.rows = onward ? p->img_rows : nullptr;
   r.out = out;
   r.tw = p->tw;
-  r.wt = p->wt;
+  r.wt = p->ramp;
   r.eps = p->eps;
   r.dimg = p->dimg;
   r.ridx = p->ridx;
@@ -613,7 +651,7 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
   r.partials = p->partials;
   r.counter = p->counter;
   r.energy = energy;
-  r.scale = scale;
+  sep_scale(p, scale, &r);
   r.planes = g.M * g.E;
   return sep_rows(g, p->dtype, mode, r, p->pdl, s);
 }
@@ -628,7 +666,7 @@ int sep_adjoint(jubik_plan* p, void* out_x, double scale, cudaStream_t s) {
     c.hmain = p->hmain;
     c.hnyq = p->hnyq;
     c.tw = p->tw;
-    c.wt = p->wt;
+    c.wt = p->ramp;
     c.slab = p->grad_slabs;
     JUBIK_TRY(sep_cols(g, p->dtype, SEP_COLS_ADJ, c, p->pdl, s));
   }
@@ -637,8 +675,8 @@ int sep_adjoint(jubik_plan* p, void* out_x, double scale, cudaStream_t s) {
   r.slab = p->grad_slabs;
   r.out = out_x;
   r.tw = p->tw;
-  r.wt = p->wt;
-  r.scale = scale;
+  r.wt = p->ramp;
+  sep_scale(p, scale, &r);
   r.planes = g.E;
   return sep_rows(g, p->dtype, SEP_GRAD, r, p->pdl, s);
 }
@@ -652,7 +690,7 @@ int sep_adjoint_of(jubik_plan* p, const void* cot, SepMode mode, void* out_x, do
     r.in = cot;
     r.rows = p->img_rows;
     r.tw = p->tw;
-    r.wt = p->wt;
+    r.wt = p->ramp;
     r.eps = p->eps;
     r.ridx = p->ridx;
     r.planes = p->g.M * p->g.E;
@@ -796,7 +834,7 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
   if (d->path != JUBIK_PATH_FUSED_UNIT && sep_supported(g, d->dtype)) {
     const SepSizes z = sep_sizes(g, d->dtype);
     const size_t mark = p->allocs.size(), bytes = p->bytes;
-    p->sep = !p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz) &&
+    p->sep = !upload_sep_tables(p) && !p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz) &&
              !p->alloc(&p->hnyq, (size_t)units * g.P * csz) &&
              !p->alloc(&p->sky_rows, z.sky_rows) && !p->alloc(&p->fwd_slabs, z.fwd_slabs) &&
              !p->alloc(&p->img_rows, z.img_rows) && !p->alloc(&p->grad_slabs, z.grad_slabs);
@@ -804,6 +842,7 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
       cudaGetLastError();
       p->release_from(mark, bytes);
       p->hmain = p->hnyq = nullptr;
+      p->gains = nullptr;
     }
   }
   if (p->path == JUBIK_PATH_FUSED) {
@@ -1012,8 +1051,8 @@ int jubik_plan_set_psf(jubik_plan* p, const void* psf, int32_t layout, int32_t e
     st = fft2_batched<double>(p->fft, p->fft, buf, nu, false, s);
     if (st) break;
     st = p->dtype == JUBIK_F32
-             ? spectra_store<float>(g, buf, u0, nu, p->hfull, p->hmain, p->hnyq, s)
-             : spectra_store<double>(g, buf, u0, nu, p->hfull, p->hmain, p->hnyq, s);
+             ? spectra_store<float>(g, buf, u0, nu, p->hfull, p->hmain, p->hnyq, p->gains, s)
+             : spectra_store<double>(g, buf, u0, nu, p->hfull, p->hmain, p->hnyq, p->gains, s);
     if (st) break;
     // sum |k| / |sum k| of each unit's window: the magnitude gain of its
     // normalised kernel, which the output bounds of the two-word sums use

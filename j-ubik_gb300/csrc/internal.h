@@ -203,7 +203,7 @@ int psf_to_cplx(const Geom& g, const void* psf, int layout, int e_broadcast, int
                 int64_t nu, double* sums, void* buf, cudaStream_t s);
 template <typename T>
 int spectra_store(const Geom& g, const void* buf, int64_t u0, int64_t nu, void* hfull,
-                  void* hmain, void* hnyq, cudaStream_t s);
+                  void* hmain, void* hnyq, const double* gains, cudaStream_t s);
 template <typename T>
 int plain_sky_patches(const Geom& g, const void* x, const void* wt, void* zs, cudaStream_t s);
 template <typename T>

@@ -78,8 +78,7 @@ __device__ __forceinline__ bool plain_quotient(float a, float x) {
 
 // a / x and b / x from one reciprocal, each quotient corrected by its residual (one
 // Newton step on the quotient, Markstein 1990).  Tested for the bits of the division over
-// that range of a and x; outside it, the division.  (Two divisions a pixel in their place:
-// 272 -> 315 us for the likelihood's rows at 1024^2 x 7 x 3.)
+// that range of a and x; outside it, the division.
 __device__ __forceinline__ void two_quotients(float a, float b, float x, float& qa, float& qb) {
   if (!plain_quotient(a, x)) {
     qa = a / x;
@@ -161,13 +160,13 @@ struct Kahan2 {
   }
 };
 
-// Two pixels (of two image rows) at once, as poisson_px.
+// Two pixels (of two image rows) at once, as poisson_px, from conv + low.
 template <typename T>
-__device__ __forceinline__ void poisson_px2(cx<T> conv, cx<T> ep, const int32_t (&d)[2],
+__device__ __forceinline__ void poisson_px2(cx<T> conv, cx<T> low, cx<T> ep, const int32_t (&d)[2],
                                             cx<T>& w_o, cx<T>& res_o, Kahan2<T>& s_lam,
                                             Kahan2<T>& s_dlog) {
   const bool a = d[0] >= 0, b = d[1] >= 0;
-  const cx<T> lam = pmul(ep, conv);
+  const cx<T> lam = pfma(ep, conv, pmul(ep, low));
   // pixels that are not read out: lam = 1 and a count of 0 enter nowhere
   const cx<T> x = mkc<T>(a ? lam.x : (T)1, b ? lam.y : (T)1);
   const cx<T> dd = mkc<T>(a ? (T)d[0] : (T)0, b ? (T)d[1] : (T)0);

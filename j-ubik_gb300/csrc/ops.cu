@@ -100,7 +100,7 @@ __global__ void k_psf_to_cplx(const T* __restrict__ psf, int layout, int e_bcast
 template <typename T>
 __global__ void k_spectra_store(const double2* __restrict__ buf, int P, int64_t u0, int64_t nu,
                                 cx<T>* __restrict__ hfull, cx<T>* __restrict__ hmain,
-                                cx<T>* __restrict__ hnyq) {
+                                cx<T>* __restrict__ hnyq, const double* __restrict__ gains) {
   const int H = P / 2;
   const int L1 = P / 16;
   const double sc = 1.0 / ((double)P * (double)P);
@@ -111,7 +111,9 @@ __global__ void k_spectra_store(const double2* __restrict__ buf, int P, int64_t 
     const int rem = (int)(i - ul * P * P);
     const int ky = rem / P, kx = rem % P;
     const double2 v = buf[i];
-    const cx<T> w = mkc<T>((T)(v.x * sc), (T)(v.y * sc));
+    const double gy = gains ? 1.0 - gains[ky] : 1.0;
+    const double sk = gains ? sc * (gy - gains[P + kx]) : sc;
+    const cx<T> w = mkc<T>((T)(v.x * sk), (T)(v.y * sk));
     const int64_t hu = u0 + ul;
     if (hfull && kx <= H) hfull[(hu * P + ky) * (H + 1) + kx] = w;
     if (hmain && kx <= H) {
@@ -119,8 +121,10 @@ __global__ void k_spectra_store(const double2* __restrict__ buf, int P, int64_t 
       if (kx == 0 || kx == H) {
         const double2 h0 = kx == 0 ? v : buf[i - H];
         const double2 hn = kx == H ? v : buf[i + H];
-        const double2 al = make_double2(0.5 * (h0.x + hn.x) * sc, 0.5 * (h0.y + hn.y) * sc);
-        const double2 be = make_double2(0.5 * (h0.x - hn.x) * sc, 0.5 * (h0.y - hn.y) * sc);
+        const double f0 = gains ? gy - gains[P] : 1.0, fn = gains ? gy - gains[P + H] : 1.0;
+        const double2 a = make_double2(f0 * h0.x, f0 * h0.y), b = make_double2(fn * hn.x, fn * hn.y);
+        const double2 al = make_double2(0.5 * (a.x + b.x) * sc, 0.5 * (a.y + b.y) * sc);
+        const double2 be = make_double2(0.5 * (a.x - b.x) * sc, 0.5 * (a.y - b.y) * sc);
         if (kx == 0)
           hmain[(hu * P + slot) * H] = mkc<T>((T)al.x, (T)al.y);
         else
@@ -1009,11 +1013,11 @@ int psf_to_cplx(const Geom& g, const void* psf, int layout, int e_broadcast, int
 
 template <typename T>
 int spectra_store(const Geom& g, const void* buf, int64_t u0, int64_t nu, void* hfull,
-                  void* hmain, void* hnyq, cudaStream_t s) {
+                  void* hmain, void* hnyq, const double* gains, cudaStream_t s) {
   const int64_t total = nu * g.P * g.P;
   k_spectra_store<T><<<grid_for(total), kBlock, 0, s>>>((const double2*)buf, g.P, u0, nu,
                                                         (cx<T>*)hfull, (cx<T>*)hmain,
-                                                        (cx<T>*)hnyq);
+                                                        (cx<T>*)hnyq, gains);
   return cuda_status(cudaGetLastError(), "k_spectra_store");
 }
 
@@ -1320,7 +1324,7 @@ int combine_words(void* hi, const void* lo, int64_t n, bool pdl, cudaStream_t s)
   template int psf_to_cplx<T>(const Geom&, const void*, int, int, int64_t, int64_t, double*,     \
                               void*, cudaStream_t);                                              \
   template int spectra_store<T>(const Geom&, const void*, int64_t, int64_t, void*, void*, void*, \
-                                cudaStream_t);                                                   \
+                                const double*, cudaStream_t);                                    \
   template int plain_sky_patches<T>(const Geom&, const void*, const void*, void*, cudaStream_t); \
   template int plain_mul_modules<T>(const Geom&, const void*, const void*, int, int, void*,      \
                                     cudaStream_t);                                               \

@@ -1,6 +1,9 @@
 // Separable response: which geometries it covers, its scratch, and the dispatch
 // by precision (the kernels are in sep_rows.cuh and sep_cols.cuh).
 #include <algorithm>
+#include <cmath>
+#include <complex>
+#include <vector>
 
 #include "sep.h"
 
@@ -23,6 +26,75 @@ SepSizes sep_sizes(const Geom& g, int dtype) {
   z.img_rows = c * (size_t)g.M * g.E * g.n * g.nx * H;
   z.grad_slabs = c * en2 * g.K * H;
   return z;
+}
+
+// The transforms' constants are rounded to FP32, so a transform and its inverse return
+// (1 + g) of a frequency, not all of it.  At side 192 g is -0.59e-7 in the mean along rows
+// and as much along columns, alike for nearly every frequency but the constant one: of the
+// back-projection's error against 64 bits (1.84e-7) 1.09e-7 was this one factor.  The PSF
+// spectra, which are computed in FP64, take the factor back before they are rounded
+// (errors before -> now at 1024^2: gradient 7.3e-7 -> 3.8e-7, metric product 3.5e-7 ->
+// 1.8e-7, back-projection 1.68e-7 -> 1.46e-7).
+// Each transform of side 16 L1 multiplies an element by one entry of the 16-point matrix,
+// one twiddle and one entry of the L1-point matrix, and its inverse by their conjugates:
+// the gain is the mean of the three squared magnitudes over the elements.
+namespace {
+using Cx = std::complex<double>;
+Cx rounded_root(int k, int N) {  // exp(-2 pi i k / N) with its parts rounded to FP32
+  const double a = -2.0 * 3.14159265358979323846 * (double)(k % N) / N;
+  return Cx((float)std::cos(a), (float)std::sin(a));
+}
+// the matrix of the N-point codelet (fft_codelets.cuh), row by row
+std::vector<Cx> codelet_matrix(int N) {
+  std::vector<Cx> m((size_t)N * N);
+  int n1 = 0;
+  switch (N) {
+    case 8: case 16: case 20: case 32: n1 = 4; break;
+    case 12: case 24: n1 = 3; break;
+    case 10: n1 = 5; break;
+    default: break;  // no factors
+  }
+  if (!n1) {
+    for (int k = 0; k < N; ++k)
+      for (int n = 0; n < N; ++n) m[k * N + n] = rounded_root(k * n, N);
+    return m;
+  }
+  const int n2 = N / n1;
+  const std::vector<Cx> a = codelet_matrix(n1), b = codelet_matrix(n2);
+  for (int i = 0; i < n2; ++i)
+    for (int k1 = 0; k1 < n1; ++k1)
+      for (int n = 0; n < n1; ++n)
+        for (int k2 = 0; k2 < n2; ++k2)
+          m[(size_t)(k1 + n1 * k2) * N + n2 * n + i] =
+              a[k1 * n1 + n] * rounded_root(i * k1, N) * b[k2 * n2 + i];
+  return m;
+}
+// squared magnitudes less one
+double excess(Cx z) { return std::norm(z) - 1.0; }
+}  // namespace
+
+void sep_gains(int P, std::vector<double>& gy, std::vector<double>& gx) {
+  const int L1 = P / 16;
+  const std::vector<Cx> a = codelet_matrix(16), b = codelet_matrix(L1);
+  std::vector<double> ea(16, 0.0), eb(L1, 0.0);  // means over a matrix row
+  for (int k = 0; k < 16; ++k)
+    for (int n = 0; n < 16; ++n) ea[k] += excess(a[k * 16 + n]) / 16;
+  for (int k = 0; k < L1; ++k)
+    for (int n = 0; n < L1; ++n) eb[k] += excess(b[k * L1 + n]) / L1;
+  // (first order: the excesses add)
+  std::vector<double> g(P);
+  gy.assign(P, 0.0);
+  gx.assign(P, 0.0);
+  for (int c = 0; c < L1; ++c)
+    for (int q = 0; q < 16; ++q) {
+      double over_n = 0.0, over_c = 0.0;
+      for (int i = 0; i < 16; ++i) over_n += excess(rounded_root(c * i, P)) / 16;
+      for (int i = 0; i < L1; ++i) over_c += excess(rounded_root(i * q, P)) / L1;
+      gy[c + L1 * q] = eb[c] + over_n + ea[q];   // columns: class c, then slot q
+      g[q + 16 * c] = ea[q] + over_c + eb[c];    // rows: slot q, then class c
+    }
+  // two real rows travel as one sequence: kx and P - kx serve both
+  for (int k = 0; k < P; ++k) gx[k] = 0.5 * (g[k] + g[(P - k) % P]);
 }
 
 bool sep_run_fits(const Geom& g, int dtype, int run) {

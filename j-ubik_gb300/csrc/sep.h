@@ -21,6 +21,8 @@
 // kx = 0 and kx = P/2 values (real for a real row) packed into column 0.
 #pragma once
 
+#include <vector>
+
 #include "internal.h"
 
 namespace jubik {
@@ -55,7 +57,7 @@ struct SepRows {
   double* partials = nullptr;
   unsigned int* counter = nullptr;
   double* energy = nullptr;
-  double scale = 1.0;
+  double scale = 1.0, scale_lo = 0.0;  // the factor's two words
   int planes = 0;              // M E, or E for SEP_SKY and SEP_GRAD
 };
 
@@ -78,6 +80,9 @@ struct SepSizes {
   size_t sky_rows, fwd_slabs, img_rows, grad_slabs;
 };
 SepSizes sep_sizes(const Geom& g, int dtype);
+// Gains less one of the column transforms (gy, by ky) and of the row transforms (gx, by kx)
+// of side P, each forward and back: P values each.
+void sep_gains(int P, std::vector<double>& gy, std::vector<double>& gx);
 // Blocks of the likelihood's row kernel at most (its partial sums).
 constexpr int kSepMaxBlocks = 2048;
 

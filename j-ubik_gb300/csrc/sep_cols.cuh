@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
       cx<T> v[16];
       tile_to_spectrum<T, L1>(buf + mine, mytw, v);
 #pragma unroll
-      for (int q = 0; q < 16; ++q) acc[q] = cadd<T>(acc[q], cmulc<T>(v[q], hv[q]));
+      for (int q = 0; q < 16; ++q) acc[q] = cmulc_add(v[q], hv[q], acc[q]);
       hb += hstep;
       if (m + 1 < k.M) load_class<T, L1, true>(hb, hv);
       if (c0) {
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
             (const cx<T>*)k.a.hnyq + (((int64_t)m * k.n2 + kp) * k.E + e) * P + 16 * it;
 #pragma unroll
         for (int q = 0; q < 16; ++q)
-          acc[q] = cadd<T>(acc[q], cmulc<T>(cconj<T>(w0[mirror_slot<L1>(it, q)]), __ldg(be + q)));
+          acc[q] = cmulc_add(cconj<T>(w0[mirror_slot<L1>(it, q)]), __ldg(be + q), acc[q]);
       }
     }
   }

@@ -26,8 +26,7 @@ __device__ __forceinline__ int sep_div(int u, int d, uint32_t mul) {
 }
 
 // a + conj(b) and (a - conj(b)) / i: twice the spectra of the two real rows of a
-// pair from the pair's transform at k and -k (the rows are halved before); and
-// their inverses
+// pair from the pair's transform at k and -k (the rows are halved before)
 template <typename T>
 __device__ __forceinline__ cx<T> split_a(cx<T> a, cx<T> b) {
   return mkc<T>(a.x + b.x, a.y - b.y);
@@ -36,13 +35,13 @@ template <typename T>
 __device__ __forceinline__ cx<T> split_b(cx<T> a, cx<T> b) {
   return mkc<T>(a.y + b.y, b.x - a.x);
 }
-template <typename T>
-__device__ __forceinline__ cx<T> join_p(cx<T> a, cx<T> b) {  // a + i b
-  return mkc<T>(a.x - b.y, a.y + b.x);
-}
-template <typename T>
-__device__ __forceinline__ cx<T> join_m(cx<T> a, cx<T> b) {  // conj(a) + i conj(b)
-  return mkc<T>(a.x + b.y, b.x - a.y);
+
+// s + e = a + b exactly, part by part (Knuth's TwoSum)
+template <typename C>
+__device__ __forceinline__ void two_sum(C a, C b, C& s, C& e) {
+  s = padd(a, b);
+  const C t = psub(s, a);
+  e = padd(psub(a, psub(s, t)), psub(b, t));
 }
 
 // Per kernel: the shared-memory opt-in raised so far and the CTAs that fit an

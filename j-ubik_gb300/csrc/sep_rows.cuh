@@ -5,7 +5,7 @@
 // travel as the real and imaginary part of one complex sequence per window.
 //   inverse half: slabs -> row spectra of the pair (sum over the slabs that
 //     cover the row, in order) -> inverse transforms -> overlap-add over the
-//     windows in shared memory (window order, compensated) -> image rows;
+//     windows in shared memory (window order, two words) -> image rows;
 //   pixels: likelihood, metric weights, readout, gradient, ...;
 //   forward half: image rows -> windows -> transforms -> row spectra.
 // Both halves run in one kernel for the likelihood and the metric, so the image
@@ -19,7 +19,7 @@
 // barriers only; the CTA meets twice per item, before and after the overlap-add.
 // The kernels are bound by the latency of the spectrum loads and by instruction
 // issue; warps that drift apart overlap the one with the other.  At 1024^2 x 7 x 3
-// the likelihood's rows move 855 MB in 268 us (3.2 TB/s).
+// the likelihood's rows move 855 MB in 289 us (3.0 TB/s).
 #include "likelihood.cuh"
 #include "sep_dev.cuh"
 
@@ -39,13 +39,15 @@ struct RowK {
   int items;                 // items in all
   uint32_t mul_dx, mul_step;  // floor(u / d) = high word of u mul (row_div)
   uint32_t div_per;
-  float scale32;
-  double scale64;
+  float scale32[2];  // the factor's two words
+  double scale64[2];
 };
-template <typename T> __device__ __forceinline__ T row_scale(const RowK& k);
-template <> __device__ __forceinline__ float row_scale<float>(const RowK& k) { return k.scale32; }
-template <> __device__ __forceinline__ double row_scale<double>(const RowK& k) {
-  return k.scale64;
+template <typename T> __device__ __forceinline__ T row_scale(const RowK& k, int word);
+template <> __device__ __forceinline__ float row_scale<float>(const RowK& k, int word) {
+  return k.scale32[word];
+}
+template <> __device__ __forceinline__ double row_scale<double>(const RowK& k, int word) {
+  return k.scale64[word];
 }
 
 // Sequences (row pair x window) a CTA holds at once: 16, or as many as fit beside
@@ -99,25 +101,45 @@ __device__ __forceinline__ void row_twiddles(const double2* tw, int q, double2& 
   b = tw[q + 1];
 }
 
-// Joins the two rows' values of kx = lane + 32 t and writes those of the pair's sequence
-// at kx and P - kx (kx = 0: the packed real kx = 0 and kx = P / 2 values).
+// Writes p = a + i b at kx = lane + 32 t and conj m, m = a - i b, at P - kx of the pair's
+// sequence (kx = 0: the packed real kx = 0 and kx = P / 2 values of a and b).
+template <typename T, int L1>
+__device__ __forceinline__ void row_store(cx<T> p, cx<T> m, const cx<T>& a, const cx<T>& b, int t,
+                                          cx<T>* wp, cx<T>* wm, int lane) {
+  const bool dc = t == 0 && lane == 0;
+  wp[34 * t] = dc ? mkc<T>(a.x, b.x) : p;
+  (dc ? wp + row_slot(8 * L1) : wm - 34 * t)[0] = dc ? mkc<T>(a.y, b.y) : cconj<T>(m);
+}
+// Joins the two rows' values.
 template <typename T, int L1>
 __device__ __forceinline__ void row_join(const cx<T> (&v)[2], int t, cx<T>* wp, cx<T>* wm,
                                          int lane) {
-  const bool dc = t == 0 && lane == 0;
-  wp[34 * t] = dc ? mkc<T>(v[0].x, v[1].x) : join_p<T>(v[0], v[1]);
-  (dc ? wp + row_slot(8 * L1) : wm - 34 * t)[0] =
-      dc ? mkc<T>(v[0].y, v[1].y) : join_m<T>(v[0], v[1]);
+  const cx<T> ib = cmul_i<T>(v[1]);
+  row_store<T, L1>(cadd<T>(v[0], ib), csub<T>(v[0], ib), v[0], v[1], t, wp, wm, lane);
+}
+// The same for sums v + lo of two words.
+template <typename T, int L1>
+__device__ __forceinline__ void row_join2(const cx<T> (&v)[2], const cx<T> (&lo)[2], int t,
+                                          cx<T>* wp, cx<T>* wm, int lane) {
+  const cx<T> ib = cmul_i<T>(v[1]), il = cmul_i<T>(lo[1]);
+  cx<T> p, pe, m, me;
+  two_sum(v[0], ib, p, pe);
+  two_sum(v[0], mkc<T>(-ib.x, -ib.y), m, me);
+  p = padd(p, padd(pe, padd(lo[0], il)));
+  m = padd(m, padd(me, psub(lo[0], il)));
+  row_store<T, L1>(p, m, padd(v[0], lo[0]), padd(v[1], lo[1]), t, wp, wm, lane);
 }
 
-// Spectra of a row pair in one window: the sum of up to N slabs, in order.  The loads of
-// three steps are issued before the first sum: with one loop for up to three slabs the
+// Spectra of a row pair in one window: the sum of up to N slabs, in FP32 in two words (in
+// FP64 the two words cost 14 % of a pass and changed its error by 0.3 %).  The loads
+// of three steps are issued before the first sum: with one loop for up to three slabs the
 // compiler interleaved loads and sums, and the likelihood's rows took 331 us at
-// 1024^2 x 7 x 3 and 381 at side 384, now 272 and 268 (2.8 -> 3.4 TB/s).
+// 1024^2 x 7 x 3 and 381 at side 384, then 272 and 268; with two words 289 and 280.
 template <typename T, int L1, int N>
 __device__ __forceinline__ void row_load(const cx<T>* p, const int (&o)[2][3], const int (&m)[2],
                                          cx<T>* wp, cx<T>* wm, int lane) {
   constexpr int H = 8 * L1, STEPS = (H + 31) / 32, G = sizeof(T) == 4 ? 3 : 1;
+  constexpr bool TWO = N > 1 && sizeof(T) == 4;
 #pragma unroll
   for (int t0 = 0; t0 < STEPS; t0 += G) {
     cx<T> z[G][2][N];
@@ -134,16 +156,38 @@ __device__ __forceinline__ void row_load(const cx<T>* p, const int (&o)[2][3], c
 #pragma unroll
     for (int t = t0; t < t0 + G && t < STEPS; ++t) {
       if (H % 32 && lane + 32 * t >= H) break;
-      cx<T> v[2];
+      cx<T> v[2], lo[2];
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
         v[b] = z[t - t0][b][0];
+        lo[b] = mkc<T>((T)0, (T)0);
 #pragma unroll
-        for (int u = 1; u < N; ++u) v[b] = cadd<T>(v[b], z[t - t0][b][u]);
+        for (int u = 1; u < N; ++u) {
+          if (TWO) {
+            cx<T> e;
+            two_sum(v[b], z[t - t0][b][u], v[b], e);
+            lo[b] = u == 1 ? e : padd(lo[b], e);
+          } else {
+            v[b] = cadd<T>(v[b], z[t - t0][b][u]);
+          }
+        }
       }
-      row_join<T, L1>(v, t, wp, wm, lane);
+      if (TWO)
+        row_join2<T, L1>(v, lo, t, wp, wm, lane);
+      else
+        row_join<T, L1>(v, t, wp, wm, lane);
     }
   }
+}
+
+// s + e = s0 + e0 + w z up to the rounding of the low words
+template <typename T>
+__device__ __forceinline__ void add_weighted(T w, cx<T> z, cx<T> s0, cx<T> e0, cx<T>& s, cx<T>& e) {
+  const cx<T> p = pmul(both<T>(w), z);
+  const cx<T> pe = pfma(both<T>(w), z, mkc<T>(-p.x, -p.y));
+  cx<T> er;
+  two_sum(s0, p, s, er);
+  e = padd(e0, padd(er, pe));
 }
 
 // DFT-L1 of class `ca` of a sequence, in place
@@ -214,7 +258,7 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
   sep_wait();
   __syncthreads();
   const cx<T>* mytw = stw + kRowTw * cls;
-  const T scale = row_scale<T>(k);
+  const T scale = row_scale<T>(k, 0), scale_lo = row_scale<T>(k, 1);
   Kahan2<T> s_lam, s_dlog;
   const int nchunk = (n * k.rp + k.seqs - 1) / k.seqs;  // > 1 only when rp == 1
 
@@ -229,7 +273,7 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
         const int hs = k.height * H;
         // the slabs that cover the pair's rows, in order (a row beyond the field: none):
         // their number and the row's offset in each
-        int lo[2], m[2], o[2][3], had = -1;
+        int lo_i[2], m[2], o[2][3], had = -1;
 #pragma unroll 1
         for (int s = q0; s < q0 + 2 && s < cnt; ++s) {
           const int r = k.rp == 1 ? 0 : s / jn, j = j0 + s - r * jn;
@@ -241,11 +285,11 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
               const int d = row0 + b - base_c, under = d - k.height + 1;
               int hi = min(k.nslab - 1, row_div(d, k.mul_step));
               if (hi + 1 == k.nslab - 1 && k.nslab * k.step - k.step - k.late <= d) ++hi;
-              lo[b] = under <= 0 ? 0 : row_div(under + k.step - 1, k.mul_step);
-              m[b] = row0 + b < nx ? hi - lo[b] + 1 : 0;
+              lo_i[b] = under <= 0 ? 0 : row_div(under + k.step - 1, k.mul_step);
+              m[b] = row0 + b < nx ? hi - lo_i[b] + 1 : 0;
 #pragma unroll
               for (int u = 0; u < 3; ++u) {
-                const int i = lo[b] + u;
+                const int i = lo_i[b] + u;
                 o[b][u] = i * hs + (d - i * k.step + (i == k.nslab - 1 ? k.late : 0)) * H;
               }
             }
@@ -265,17 +309,20 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
 #pragma unroll 1
             for (int t = 0; t < (H + 31) / 32; ++t) {
               if (H % 32 && lane + 32 * t >= H) break;
-              cx<T> v[2];
+              cx<T> v[2], lo[2];
 #pragma unroll
               for (int b = 0; b < 2; ++b) {
-                v[b] = mkc<T>((T)0, (T)0);
+                v[b] = lo[b] = mkc<T>((T)0, (T)0);
                 const int step = hs - k.step * H, first = o[b][0];
 #pragma unroll 4
-                for (int u = 0; u < m[b]; ++u)
-                  v[b] = cadd<T>(v[b], p[first + u * step + 32 * t +
-                                         (u && lo[b] + u == k.nslab - 1 ? late : 0)]);
+                for (int u = 0; u < m[b]; ++u) {
+                  cx<T> e;
+                  two_sum(v[b], p[first + u * step + 32 * t +
+                                  (u && lo_i[b] + u == k.nslab - 1 ? late : 0)], v[b], e);
+                  lo[b] = padd(lo[b], e);
+                }
               }
-              row_join<T, L1>(v, t, wp, wm, lane);
+              row_join2<T, L1>(v, lo, t, wp, wm, lane);
             }
           }
         }
@@ -318,7 +365,10 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
           for (int xb = tid; xb < ny; xb += U * NT) {
             T f[U][2];
             int32_t ix[U][2];
-            if (MODE != SEP_GRAD) {
+            if (MODE == SEP_GRAD) {
+#pragma unroll
+              for (int u = 0; u < U; ++u) f[u][0] = f[u][1] = (T)1;
+            } else {
 #pragma unroll
               for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -341,88 +391,92 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
               const int x = xb + u * NT;
               if (x >= ny) break;
               const uint32_t e = xwin[x];
-              cx<T> sum;
+              cx<T> sum, rest;  // the two words of the sum over the windows
               if (k.few) {
-                // compensated sum of up to four windows' values, in window order
+                // up to four windows' values, in window order
                 const cx<T>* w = wbuf + (e & 0xffffu);
                 const int cw = (int)(e >> 16) & 15, S = WP - k.dx;
                 const cx<T> z = mkc<T>((T)0, (T)0);
-                cx<T> z0 = cw > 0 ? w[0] : z, z1 = cw > 1 ? w[S] : z;
-                cx<T> z2 = cw > 2 ? w[2 * S] : z;
+                const cx<T> z0 = cw > 0 ? w[0] : z, z1 = cw > 1 ? w[S] : z;
+                const cx<T> z2 = cw > 2 ? w[2 * S] : z;
                 if (GRAD) {  // the windows' column weights
                   const T* wx0 = wt + (e >> 20);
                   const T g0 = cw > 0 ? wx0[0] : (T)0, g1 = cw > 1 ? wx0[-k.dx] : (T)0;
                   const T g2 = cw > 2 ? wx0[-2 * k.dx] : (T)0;
-                  z0 = mkc<T>(g0 * z0.x, g0 * z0.y);
-                  z1 = mkc<T>(g1 * z1.x, g1 * z1.y);
-                  z2 = mkc<T>(g2 * z2.x, g2 * z2.y);
-                }
-                const cx<T> t = padd(z0, z1);
-                const cx<T> y = psub(z2, psub(psub(t, z0), z1));
-                sum = padd(t, y);
-                if (cw > 3) {
-                  cx<T> z3 = w[3 * S];
-                  if (GRAD) {
-                    const T g3 = wt[(int)(e >> 20) - 3 * k.dx];
-                    z3 = mkc<T>(g3 * z3.x, g3 * z3.y);
+                  add_weighted<T>(g0, z0, z, z, sum, rest);
+                  add_weighted<T>(g1, z1, sum, rest, sum, rest);
+                  add_weighted<T>(g2, z2, sum, rest, sum, rest);
+                  if (cw > 3)
+                    add_weighted<T>(wt[(int)(e >> 20) - 3 * k.dx], w[3 * S], sum, rest, sum, rest);
+                } else {
+                  cx<T> er;
+                  two_sum(z0, z1, sum, rest);
+                  two_sum(sum, z2, sum, er);
+                  rest = padd(rest, er);
+                  if (cw > 3) {
+                    two_sum(sum, w[3 * S], sum, er);
+                    rest = padd(rest, er);
                   }
-                  sum = cadd<T>(sum, csub<T>(z3, csub<T>(csub<T>(sum, t), y)));
                 }
               } else {
                 int j = (int)(e >> 16), jend = j + (int)(e & 0xffffu);
                 j = max(j, j0);
                 jend = min(jend, j0 + jn);
-                Kahan<T> re, im;
+                sum = rest = mkc<T>((T)0, (T)0);
                 if (ch > 0) {
-                  const cx<T> s = line[x], cc = comp[x];
-                  re.s = s.x;
-                  im.s = s.y;
-                  re.c = cc.x;
-                  im.c = cc.y;
+                  sum = line[x];
+                  rest = comp[x];
                 }
                 const cx<T>* w = wbuf + (j - j0) * WP + x + off - base_c;
                 for (int st = j * k.dx; j < jend; ++j, st += k.dx, w += WP) {
                   const int s0 = min(st, k.sc_max);
-                  cx<T> z = w[-s0];
+                  const cx<T> z = w[-s0];
                   if (GRAD) {
-                    const T ww = wt[x - base_c - s0];
-                    z = mkc<T>(ww * z.x, ww * z.y);
+                    add_weighted<T>(wt[x - base_c - s0], z, sum, rest, sum, rest);
+                  } else {
+                    cx<T> er;
+                    two_sum(sum, z, sum, er);
+                    rest = padd(rest, er);
                   }
-                  re.add(z.x);
-                  im.add(z.y);
                 }
-                sum = mkc<T>(re.s, im.s);
                 if (!last) {
                   line[x] = sum;
-                  comp[x] = mkc<T>(re.c, im.c);
+                  comp[x] = rest;
                   continue;
                 }
               }
+              // the scaled sum in two words: v, and what v lacks
               const cx<T> v = pmul(both<T>(scale), sum);
+              const cx<T> vl = pfma(both<T>(scale), rest,
+                                    pfma(both<T>(scale_lo), sum,
+                                         pfma(both<T>(scale), sum, mkc<T>(-v.x, -v.y))));
               const int64_t p = px0 + x;
               if (MODE == SEP_LIKE) {
                 cx<T> wgt, res;
-                poisson_px2<T>(v, mkc<T>(f[u][0], f[u][1]), ix[u], wgt, res, s_lam, s_dlog);
+                poisson_px2<T>(v, vl, mkc<T>(f[u][0], f[u][1]), ix[u], wgt, res, s_lam, s_dlog);
                 __stcs((T*)a.wts + p, wgt.x);
                 if (two) __stcs((T*)a.wts + p + ny, wgt.y);
                 if (FWD) line[r * ny + x] = pmul(both<T>((T)0.5), res);
-              } else if (MODE == SEP_METRIC) {
-                if (FWD)
-                  line[r * ny + x] = mkc<T>((T)0.5 * (f[u][0] * v.x),
-                                            two ? (T)0.5 * (f[u][1] * v.y) : (T)0);
               } else {
+                const cx<T> fv = mkc<T>(f[u][0], f[u][1]);
+                // (factor) (v + vl), rounded once
+                const cx<T> fp = pfma(fv, v, pmul(fv, vl));
+                if (MODE == SEP_METRIC) {
+                  if (FWD) line[r * ny + x] = mkc<T>((T)0.5 * fp.x, two ? (T)0.5 * fp.y : (T)0);
+                } else {
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                  if (b && !two) break;
-                  const int64_t pb = p + (int64_t)b * ny;
-                  const T vb = b ? v.y : v.x;
-                  if (MODE == SEP_GRAD || k.mode == SEP_IMAGE) {
-                    ((T*)a.out)[pb] = vb;
-                  } else if (k.mode == SEP_READOUT) {
-                    if (ix[u][b] >= 0) ((T*)a.out)[ix[u][b]] = eps ? f[u][b] * vb : vb;
-                  } else {  // SEP_WEIGHTS
-                    const T ep = f[u][b];
-                    ((T*)a.wts)[pb] = ix[u][b] < 0 ? (T)0 : (ep * ep) / (ep * vb);
+                  for (int b = 0; b < 2; ++b) {
+                    if (b && !two) break;
+                    const int64_t pb = p + (int64_t)b * ny;
+                    const T vb = b ? fp.y : fp.x;
+                    if (MODE == SEP_GRAD || k.mode == SEP_IMAGE) {
+                      ((T*)a.out)[pb] = vb;
+                    } else if (k.mode == SEP_READOUT) {
+                      if (ix[u][b] >= 0) ((T*)a.out)[ix[u][b]] = vb;
+                    } else {  // SEP_WEIGHTS
+                      const T ep = f[u][b];
+                      ((T*)a.wts)[pb] = ix[u][b] < 0 ? (T)0 : (ep * ep) / vb;
+                    }
                   }
                 }
               }
@@ -603,8 +657,10 @@ int dispatch_rows(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaS
   k.sr_max = g.sr_max;
   k.sc_max = g.sc_max;
   k.K = g.K;
-  k.scale32 = (float)a.scale;
-  k.scale64 = a.scale;
+  k.scale64[0] = a.scale;
+  k.scale64[1] = a.scale_lo;
+  k.scale32[0] = (float)a.scale;
+  k.scale32[1] = (float)(a.scale - (double)k.scale32[0] + a.scale_lo);
   const bool grad = mode == SEP_GRAD;
   k.nslab = g.n / a.slab_run;
   k.step = g.dx * a.slab_run;
