@@ -20,7 +20,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libjubik_gb300.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["fused.cu", "plain_fft.cu", "ops.cu", "api.cu", "noalloc.cu",
+SOURCES = ["fused.cu", "plain_fft.cu", "plain_cols.cu", "ops.cu", "api.cu", "noalloc.cu",
            "sampling.cu", "psf_interp.cu", "sky_cf.cu", "sep.cu", "sep_rows_f32.cu",
            "sep_rows_f64.cu", "sep_cols_f32.cu", "sep_cols_f64.cu"]
 

@@ -397,6 +397,13 @@ int adj_terms_log2(const Geom& g) {
   return terms_log2(per * per * g.M);
 }
 
+// row pass of the unfused path's 2-D transforms over batch P x P arrays
+template <typename T>
+int plain_rows(jubik_plan* p, void* data, int64_t batch, bool inverse, cudaStream_t s) {
+  const int64_t P = p->g.P;
+  return fft_batched<T>(p->fft, data, batch * P, (int)P, P * P, P, 1, inverse, 1.0, s);
+}
+
 int do_forward(jubik_plan* p, const void* x, void* out, void* out_lo, double scale,
                cudaStream_t s, void* also_zero = nullptr, int64_t also_zero_bytes = 0,
                bool* zeroed = nullptr, SkyView view = SkyView()) {
@@ -416,6 +423,7 @@ int do_forward(jubik_plan* p, const void* x, void* out, void* out_lo, double sca
   if (p->path == JUBIK_PATH_FUSED) {
     FusedLaunch a{x, out, p->hmain, p->hnyq, p->tw, p->wt, scale, p->spec};
     a.pdl = p->pdl;
+    a.fwd_run = p->fwd_run;
     a.in_ps = view.ps;
     a.in_rs = view.rs;
     a.in_exp = view.exp;
@@ -462,6 +470,24 @@ int do_forward(jubik_plan* p, const void* x, void* out, void* out_lo, double sca
   }
   Phase ph(p, 0, s);
   const bool f32 = p->dtype == JUBIK_F32;
+  if (plain_cols_supported(g.P)) {
+    // row pass over the weighted sky windows; per module chunk: column stage
+    // with the PSF product, inverse row pass, overlap gather
+    const void* tw = f32 ? p->fft.tw32 : p->fft.tw64;
+    JUBIK_TRY(f32 ? fft_rows_windows<float>(p->fft, g, x, false, p->wt, 0, 1, p->zs, s)
+                  : fft_rows_windows<double>(p->fft, g, x, false, p->wt, 0, 1, p->zs, s));
+    for (int m0 = 0; m0 < g.M; m0 += p->zu_modules) {
+      const int nm = std::min(p->zu_modules, g.M - m0);
+      JUBIK_TRY(f32 ? plain_cols_forward<float>(g, p->zs, p->hfull, tw, m0, nm, p->zu, s)
+                    : plain_cols_forward<double>(g, p->zs, p->hfull, tw, m0, nm, p->zu, s));
+      const int64_t batch = (int64_t)nm * plain_pairs(g);
+      JUBIK_TRY(f32 ? plain_rows<float>(p, p->zu, batch, true, s)
+                    : plain_rows<double>(p, p->zu, batch, true, s));
+      JUBIK_TRY(f32 ? plain_overlap_gather<float>(g, p->zu, m0, nm, scale, out, s)
+                    : plain_overlap_gather<double>(g, p->zu, m0, nm, scale, out, s));
+    }
+    return JUBIK_OK;
+  }
   JUBIK_TRY(f32 ? plain_sky_patches<float>(g, x, p->wt, p->zs, s)
                 : plain_sky_patches<double>(g, x, p->wt, p->zs, s));
   JUBIK_TRY(f32 ? fft2_batched<float>(p->fft, p->fft, p->zs, plain_pairs(g), false, s)
@@ -537,6 +563,26 @@ int do_adjoint(jubik_plan* p, const void* cot, void* out_x, void* out_lo, double
   }
   Phase ph(p, 1, s);
   const bool f32 = p->dtype == JUBIK_F32;
+  if (plain_cols_supported(g.P)) {
+    // per module chunk: row pass over the cotangent windows, column stage summing
+    // the conjugate-PSF products over modules; then the inverse row pass and the
+    // gradient gather
+    const void* tw = f32 ? p->fft.tw32 : p->fft.tw64;
+    for (int m0 = 0; m0 < g.M; m0 += p->zu_modules) {
+      const int nm = std::min(p->zu_modules, g.M - m0);
+      const bool first = m0 == 0, last = m0 + nm == g.M;
+      JUBIK_TRY(f32 ? fft_rows_windows<float>(p->fft, g, cot, true, nullptr, m0, nm, p->zu, s)
+                    : fft_rows_windows<double>(p->fft, g, cot, true, nullptr, m0, nm, p->zu, s));
+      JUBIK_TRY(f32 ? plain_cols_adjoint<float>(g, p->zu, p->hfull, tw, m0, nm, first, last,
+                                                p->zs, s)
+                    : plain_cols_adjoint<double>(g, p->zu, p->hfull, tw, m0, nm, first, last,
+                                                 p->zs, s));
+    }
+    JUBIK_TRY(f32 ? plain_rows<float>(p, p->zs, plain_pairs(g), true, s)
+                  : plain_rows<double>(p, p->zs, plain_pairs(g), true, s));
+    return f32 ? plain_grad_gather<float>(g, p->zs, p->wt, scale, out_x, s)
+               : plain_grad_gather<double>(g, p->zs, p->wt, scale, out_x, s);
+  }
   for (int m0 = 0; m0 < g.M; m0 += p->zu_modules) {
     const int nm = std::min(p->zu_modules, g.M - m0);
     JUBIK_TRY(f32 ? plain_cot_patches<float>(g, cot, m0, nm, p->zu, s)
@@ -592,7 +638,8 @@ bool sets_forward_run(const jubik_plan* p) {
 }
 // Patches per run of the forward's columns: the setting, or the library's choice.
 int forward_run_of(const jubik_plan* p) {
-  if (!p->sep) return 1;
+  if (!p->sep)
+    return sets_forward_run(p) ? fused_fwd_run_len(p->g, p->dtype, p->fwd_run) : 1;
   if (sets_forward_run(p) && p->fwd_run) return p->fwd_run;
   return sep_auto_run(p->g, p->dtype);
 }
@@ -706,6 +753,13 @@ int sep_aligned(const jubik_plan* p, const void* out) {
     return JUBIK_ERR_INVALID_ARGUMENT;
   }
   return JUBIK_OK;
+}
+
+// JUBIK_SEPARABLE=0 (read at plan creation, for debugging): plans take the kernels they
+// would take where the separable ones do not cover their field.
+bool separable_wanted() {
+  const char* env = std::getenv("JUBIK_SEPARABLE");
+  return !(env && env[0] == '0' && env[1] == 0);
 }
 
 int need(bool ok, const char* what) {
@@ -831,7 +885,7 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
   if ((st = fft1d_init(&p->fft, g.P))) return fail(st);
   p->tw = p->dtype == JUBIK_F32 ? p->fft.tw32 : p->fft.tw64;
   // the separable kernels where they cover the FFT side and their scratch fits
-  if (d->path != JUBIK_PATH_FUSED_UNIT && sep_supported(g, d->dtype)) {
+  if (d->path != JUBIK_PATH_FUSED_UNIT && separable_wanted() && sep_supported(g, d->dtype)) {
     const SepSizes z = sep_sizes(g, d->dtype);
     const size_t mark = p->allocs.size(), bytes = p->bytes;
     p->sep = !upload_sep_tables(p) && !p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz) &&
@@ -949,7 +1003,8 @@ int jubik_plan_set_forward_run(jubik_plan* p, int32_t run_len) {
     set_error("set_forward_run: run length %d is not 0, 1, 2 or 4", run_len);
     return JUBIK_ERR_INVALID_ARGUMENT;
   }
-  if (run_len > 1 && !(sets_forward_run(p) && sep_run_fits(p->g, p->dtype, run_len))) {
+  if (run_len > 1 && !(sets_forward_run(p) && (p->sep ? sep_run_fits(p->g, p->dtype, run_len)
+                                                    : fused_fwd_run_len(p->g, p->dtype, run_len) > 0))) {
     set_error("set_forward_run: runs of %d patches need the module-shared FP32 kernels at FFT "
               "side 192 with 64-pixel strides, a 32-pixel margin and %d | n", run_len, run_len);
     return JUBIK_ERR_UNSUPPORTED;

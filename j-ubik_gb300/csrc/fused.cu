@@ -87,9 +87,10 @@ struct Args {
   // the patch a CTA continues (one slot per CTA of the loop grid `loop_grid`)
   void* spill;
   int loop_grid;
-  // floor(u / d) for d = M, n^2 and n as one multiply-high by these
+  int run_len;  // run-ordered forward: patches per run (2 or 4)
+  // floor(u / d) for d = M, n^2, n and n / run_len as one multiply-high by these
   // constants (mulhi_divisor); 0: divide
-  uint32_t div_M, div_n2, div_n;
+  uint32_t div_M, div_n2, div_n, div_nq;
 };
 
 // floor(u / d) for 0 <= u: with mul = floor(2^32 / d) + 1 the high word of u mul
@@ -1430,6 +1431,164 @@ __global__ void __launch_bounds__(Tr<T, P>::NT) k_fwd_from_spec(Src src, int uni
   }
 }
 
+// ---- forward of aligned geometries in runs of vertically adjacent patches
+// When P = 3 dx with dx = 64 and margin dx / 2, a patch's P x P output covers
+// exactly three block rows of dx field rows (i - 1, i, i + 1 for patch row i),
+// and the staging chunks of the output stage (32 pair rows) are those block
+// rows.  A CTA then takes runs of a.run_len (2 or 4) vertically adjacent
+// patches of one module and adds the block rows they share in TMEM, in patch
+// order, before they leave the CTA: each block row of a run is reduced into the
+// image once (as an exact two-word sum), 6 block rows per run of 4 patches
+// instead of 12.  The modules of a run are consecutive work items, which
+// neighbouring CTAs run at the same time, so the shared sky spectra still meet
+// in L2.  Longer runs mean fewer reductions but fewer work items: the run
+// length is a schedule choice (auto_run_len, or set per plan).
+constexpr int kRunCols = 96;  // TMEM columns of one pending block row (per lane)
+
+// Output stage of patch s (0 .. run_len - 1) of a run: chunk c is block row
+// i - 1 + c.  Thread (warp w, lane) owns, in every chunk, the warp tiles of
+// the overlap-add (8 pair rows x 16 columns; the tile row tau = 0..3 gives pair
+// rows 8 tau + lane / 4, columns 16 w + 4 (lane % 4) .. + 4): 32 values, kept for
+// the pending block rows in its TMEM lane 32 (w % 4) + lane, columns
+// 96 slot + 32 (w / 4) .. + 32 (slot = block row % 2).
+template <typename T, int P>
+__device__ __forceinline__ void stage_output_run(Unit<T, P>& U, const Args& a,
+                                                 const Split2<T>& sp, uint32_t tbase, int s) {
+  static_assert(sizeof(T) == 4 && P == 192, "runs cover FP32 patches of side 192");
+  using R = Tr<T, P>;
+  constexpr int L1 = R::L1, TP = R::TP, CH = R::CH;
+  const T scale = (T)a.scale;
+  const uint32_t tl = tbase + ((uint32_t)(32 * (U.warp & 3)) << 16) +
+                      (uint32_t)((U.warp >> 2) * 32);
+  const int64_t plane = ((int64_t)U.m * a.E + U.e) * U.npix;
+  T* __restrict__ dst = (T*)a.out + plane;
+  T* __restrict__ dlo = (T*)a.out_lo + plane;
+  const int x = 16 * U.warp + 4 * (U.lane & 3);
+  const int col = U.cb + x;  // a multiple of 4: the group lies wholly in or out of the field
+  const bool col_in = col >= 0 && col + 4 <= a.ny;
+  const int i = U.k % a.n;  // patch row
+  for (int c = 0; c < 3; ++c) {
+    const int j0 = c * CH;
+    cx<T>* stg = (c & 1) ? U.tile + (j0 - CH) * TP : U.stg;
+    {  // inverse variant-A phase 2 of the chunk's 32 pair rows -> natural order
+      const int jj = U.lane;
+      const cx<T>* srcr = U.tile + (j0 + jj) * TP + 16 * U.cls;
+      cx<T> v[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) v[q] = q ? cmulc<T>(srcr[q], U.wq[q]) : srcr[q];
+      Dft<16, true, T>::run(v);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) stg[jj * TP + U.cls + L1 * q] = v[q];
+    }
+    __syncthreads();
+    T v[32];  // tile row tau: v[8 tau .. + 4] row 2 jj, v[8 tau + 4 .. + 4] row 2 jj + 1
+#pragma unroll
+    for (int tau = 0; tau < 4; ++tau) {
+      const cx<T>* sq = stg + (8 * tau + (U.lane >> 2)) * TP + x;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const cx<T> z = sq[t];
+        v[8 * tau + t] = scale * z.x;
+        v[8 * tau + 4 + t] = scale * z.y;
+      }
+    }
+    const int br = i - 1 + c;  // block row of the field
+    const uint32_t ta = tl + (uint32_t)(((br + 2) & 1) * kRunCols);
+    // warp-uniform: pending rows exist from the run's previous patch; a row
+    // leaves the CTA once no later patch of the run adds to it
+    if (s > 0 && c < 2) {
+      uint32_t r[32];
+      tmem_ld32(ta, r);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(r[j]);
+    }
+    if (c == 0 || s == a.run_len - 1) {
+      if (col_in) {
+#pragma unroll
+        for (int tau = 0; tau < 4; ++tau) {
+          const int row = U.rb + 2 * (j0 + 8 * tau + (U.lane >> 2));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (row + h < 0 || row + h >= a.nx) continue;
+            const int64_t o = (int64_t)(row + h) * a.ny + col;
+            const int q = 8 * tau + 4 * h;
+            acc4<true>((float*)(dst + o), (float*)(dlo + o), (const Split2<float>&)sp, v[q],
+                       v[q + 1], v[q + 2], v[q + 3]);
+          }
+        }
+      }
+    } else {
+      uint32_t r[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(v[j]);
+      tmem_st32(ta, r);
+    }
+  }
+  tmem_wait_st();
+}
+
+// Work item w of the run-ordered forward: module fastest, then the run q of
+// run_len patch rows, the patch column j, the energy e.  Returns unit (w, s).
+__device__ __forceinline__ int run_unit(const Args& a, int w, int s) {
+  const int nq = a.n / a.run_len;
+  int t = div_by(w, a.M, a.div_M);
+  const int m = w - t * a.M;
+  const int t2 = div_by(t, nq, a.div_nq);
+  const int q = t - t2 * nq;
+  t = t2;
+  const int e = div_by(t, a.n, a.div_n), j = t - e * a.n;
+  const int k = a.run_len * q + s + a.n * j;
+  return ((e * a.n * a.n + k) * a.M + m);
+}
+
+template <typename T, int P>
+__global__ void __launch_bounds__(Tr<T, P>::NT) k_fwd_run(Args a, int items) {
+  using R = Tr<T, P>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned long long s_slot;
+  __shared__ uint32_t s_tmem;
+  pdl_trigger();
+  int w = blockIdx.x, s = 0;
+  Unit<T, P> U;
+  U.init(a, smem_raw, true, run_unit(a, w, 0));
+  prefetch_unit(U.hmain, sizeof(cx<T>) * P * R::H, U.hnyq, sizeof(cx<T>) * P);
+  if (U.warp == 0) tmem_alloc(&s_tmem, 2 * kRunCols <= 256 ? 256 : 512);
+  tmem_fence_before_sync();
+  __syncthreads();
+  tmem_fence_after_sync();
+  const uint32_t tbase = s_tmem;
+  pdl_wait();
+  if (threadIdx.x == 32) prefetch_l2(U.spec, sizeof(cx<T>) * P * R::H);
+  const Split2<T> sp = output_splitter<T>(a, &s_slot);
+  for (;;) {
+    const int sn = s + 1 < a.run_len ? s + 1 : 0;
+    const int wn = s + 1 < a.run_len ? w : w + (int)gridDim.x;
+    const bool more = wn < items;
+    stage_mid<T, P, MID_FROM_SPEC, false>(U);
+    __syncthreads();
+    stage_invB<T, P, 0>(U, U.tid, R::NT);
+    __syncthreads();
+    stage_combine<T, P>(U, 0, R::H);
+    __syncthreads();
+    if (more) {  // the output stage's reductions leave HBM reads free
+      Unit<T, P> N;
+      N.geom(a, smem_raw, true, run_unit(a, wn, sn));
+      prefetch_unit(N.hmain, sizeof(cx<T>) * P * R::H, N.hnyq, sizeof(cx<T>) * P);
+      if (threadIdx.x == 32) prefetch_l2(N.spec, sizeof(cx<T>) * P * R::H);
+    }
+    stage_output_run<T, P>(U, a, sp, tbase, s);
+    if (!more) break;
+    __syncthreads();  // the output stage's last staging reads before the next mid writes
+    w = wn;
+    s = sn;
+    U.geom(a, smem_raw, true, run_unit(a, w, s));
+  }
+  tmem_fence_before_sync();
+  __syncthreads();
+  tmem_fence_after_sync();
+  if (U.warp == 0) tmem_dealloc(tbase, 2 * kRunCols <= 256 ? 256 : 512);
+}
+
 // Shared memory of the ordered adjoint beyond the tile: column 0's two terms
 // and running sum (3 P complex values).
 template <typename T, int P>
@@ -1670,6 +1829,7 @@ void set_div_consts(Args& a, int64_t units) {
   a.div_M = mulhi_divisor(a.M, bound);
   a.div_n2 = mulhi_divisor((int64_t)a.n * a.n, bound);
   a.div_n = mulhi_divisor(a.n, bound);
+  a.div_nq = a.run_len > 0 ? mulhi_divisor(a.n / a.run_len, bound) : 0;
 }
 
 Args make_args(const Geom& g, const FusedLaunch& f, int which, size_t esz) {
@@ -1720,6 +1880,7 @@ Args make_args(const Geom& g, const FusedLaunch& f, int which, size_t esz) {
   a.bnd_out = (unsigned long long*)f.bnd_out;
   a.spill = f.spill;
   a.loop_grid = (int)f.loop_grid;
+  a.run_len = 0;
   set_div_consts(a, g.units());
   return a;
 }
@@ -1770,6 +1931,7 @@ int ensure_smem_attrs() {
     JUBIK_TRY(set_smem(k_fwd_from_spec<T, P, ProblemList>, smem));
     JUBIK_TRY(set_smem(k_adj_to_spec_ord<T, P>, ord_smem_bytes<T, P>()));
     JUBIK_TRY(set_smem(k_adj_to_spec_ord_list<T, P>, ord_smem_bytes<T, P>()));
+    if constexpr (sizeof(T) == 4 && P == 192) JUBIK_TRY(set_smem(k_fwd_run<T, P>, smem));
     attr_set[dev] = true;
   }
   return JUBIK_OK;
@@ -1806,6 +1968,39 @@ int launch_pdl(KernelT kern, int64_t grid, bool pdl, cudaStream_t s, ArgsT... ar
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cuda_status(cudaLaunchKernelEx(&cfg, kern, args...), "fused kernel launch");
+}
+
+// Geometries whose patch outputs share whole block rows of 64 field rows (see
+// k_fwd_run): P = 192 from 64-row strides and a 32-pixel margin, a field of
+// whole strides (no clamped start), and runs of run_len (2 or 4) patch rows.
+inline bool run_geometry(const Geom& g, int run_len) {
+  return (run_len == 2 || run_len == 4) && g.P == 192 && g.dx == 64 && g.margin == 32 &&
+         g.nx == g.n * 64 && g.ny == g.n * 64 && g.n % run_len == 0 && g.M >= 2;
+}
+
+// Run length of the module-shared forward when the plan leaves it to the
+// library: the one whose busiest CTA does the least work.  A CTA of the
+// 152-CTA loop processes ceil(items / G) items of run_len units each, and a
+// unit inside a run costs about 0.87 (runs of 4) or 0.93 (runs of 2) of one
+// reduced on its own (fewer block-row reductions; measured forward times at
+// 768^2 and 1024^2 x 7 modules x 3 energies, where every choice gives the
+// busiest CTA the same number of units).
+inline int auto_run_len(const Geom& g) {
+  const int64_t G = sm_count(), U = g.units();
+  int best = 1;
+  double best_cost = (double)((U + G - 1) / G);
+  const int cand[2] = {2, 4};
+  const double f[2] = {0.93, 0.87};
+  for (int i = 0; i < 2; ++i) {
+    if (!run_geometry(g, cand[i])) continue;
+    const int64_t items = U / cand[i];
+    const double cost = (double)((items + G - 1) / G) * cand[i] * f[i];
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = cand[i];
+    }
+  }
+  return best;
 }
 
 // Grid of the ordered adjoint over g's units (its CTAs' unit ranges and spill
@@ -1849,6 +2044,17 @@ int launch_one(const Geom& g, const FusedLaunch& f, int which, cudaStream_t s) {
     case FUSED_FWD_FROM_SPEC:
       if (!need(f.out_lo && f.bnd_in && f.bnd_n == patches, "low-word plane or input bound"))
         return JUBIK_ERR_STATE;
+      if constexpr (sizeof(T) == 4 && P == 192) {
+        const int r = f.fwd_run > 0 ? f.fwd_run : auto_run_len(g);
+        if (run_geometry(g, r)) {
+          const int64_t items = units / r;
+          Args ar = a;
+          ar.run_len = r;
+          set_div_consts(ar, units);
+          return launch_pdl<T, P>(k_fwd_run<T, P>, loop_grid<T, P>(k_fwd_run<T, P>, items),
+                                  f.pdl, s, ar, (int)items);
+        }
+      }
       return launch_pdl<T, P>(k_fwd_from_spec<T, P, OneProblem>,
                               loop_grid<T, P>(k_fwd_from_spec<T, P, OneProblem>, units), f.pdl,
                               s, OneProblem{a}, (int)units);
@@ -2061,6 +2267,16 @@ int64_t fused_adj_grid(const Geom& g, int dtype) {
   if ((dtype == JUBIK_F32 ? ensure_attrs_dispatch<float>(g.P) : ensure_attrs_dispatch<double>(g.P)))
     return 0;
   return dtype == JUBIK_F32 ? ord_grid_dispatch<float>(g) : ord_grid_dispatch<double>(g);
+}
+
+// Run length the module-shared forward of geometry g uses for a request
+// (0: the library's choice): 2 or 4 for the run-ordered kernel, 1 for one
+// unit at a time.  Returns -1 for a request the geometry cannot take.
+int fused_fwd_run_len(const Geom& g, int dtype, int requested) {
+  const bool fits = dtype == JUBIK_F32 && g.P == 192;
+  if (requested == 0) return fits ? auto_run_len(g) : 1;
+  if (requested == 1) return 1;
+  return fits && run_geometry(g, requested) ? requested : -1;
 }
 
 // CTAs of the ordered adjoint over a list of problems at FFT side P that the

@@ -87,6 +87,16 @@ template <typename T>
 int fft2_batched(const Fft1D& fh, const Fft1D& fw, void* data, int64_t batch, bool inverse,
                  cudaStream_t s);
 
+// Forward row pass of the unfused path reading its rows from the images: pair
+// j's row y holds row y of patch 2j's and 2j+1's P x P windows (real and
+// imaginary parts), zero outside the field.  module_axis: img is (M, E, nx, ny)
+// and the nm modules from m0 are transformed; else img is (E, nx, ny) (nm = 1).
+// wt != nullptr applies the sky's window weights.  out: (nm, pairs, P, P).
+// FFT sides P = 16 L1 with L1 in {10, 12, 16, 20, 24, 32}.
+template <typename T>
+int fft_rows_windows(const Fft1D& f, const Geom& g, const void* img, bool module_axis,
+                     const void* wt, int m0, int nm, void* out, cudaStream_t s);
+
 // ------------------------------------------------------------------ fused path
 bool fused_supported(int P, int dtype);
 size_t fused_smem_bytes(int P, int dtype);
@@ -123,10 +133,16 @@ struct FusedLaunch {
   // and its grid (fused_adj_grid)
   void* spill = nullptr;
   int64_t loop_grid = 0;
+  // module-shared forward: patches per run of the run-ordered kernel (0: the
+  // library's choice, 1: one unit at a time; see fused_fwd_run_len)
+  int fwd_run = 0;
 };
 // CTAs of the ordered module-shared adjoint for geometry g (0 where the fused
 // path does not cover g.P): the count of its unit ranges and spill slots.
 int64_t fused_adj_grid(const Geom& g, int dtype);
+// Run length of the module-shared forward for a request (0 = the library's
+// choice): 1, 2 or 4, or -1 where geometry g cannot take the request.
+int fused_fwd_run_len(const Geom& g, int dtype, int requested);
 // CTAs of the ordered module-shared adjoint at FFT side P that fit on the GPU
 // at once (0 where the fused path does not cover P).
 int64_t fused_ord_capacity(int P, int dtype);
@@ -220,6 +236,21 @@ int plain_mulconj_accum(const Geom& g, const void* zu, const void* hfull, int m0
 template <typename T>
 int plain_grad_gather(const Geom& g, const void* zs, const void* wt, double scale, void* out,
                       cudaStream_t s);
+
+// Column stage of the unfused path fused with the PSF product (plain_cols.cu),
+// for FFT sides P = 16 L1 with L1 in {10, 12, 16, 20, 24, 32}.  Forward: zs
+// holds the row-transformed sky pairs; zu gets, per module of the chunk
+// [m0, m0 + nm), the products with their columns transformed back (the inverse
+// row pass follows).  Adjoint: zu holds the chunk's row-transformed cotangent
+// pairs; zs gets their conjugate-PSF products summed over modules, added to
+// the sum of earlier chunks (first: none) and transformed back (last).
+bool plain_cols_supported(int P);
+template <typename T>
+int plain_cols_forward(const Geom& g, const void* zs, const void* hfull, const void* tw, int m0,
+                       int nm, void* zu, cudaStream_t s);
+template <typename T>
+int plain_cols_adjoint(const Geom& g, const void* zu, const void* hfull, const void* tw, int m0,
+                       int nm, bool first, bool last, void* zs, cudaStream_t s);
 
 template <typename T>
 int slice_patches_op(const void* x, int64_t batch, int nx, int ny, int n, int dr, void* out,
