@@ -43,15 +43,19 @@ enum jubik_status {
 
 enum jubik_dtype { JUBIK_F32 = 0, JUBIK_F64 = 1 };
 
+/* Fields too wide for the separable row kernels, and plans that do not fit in device memory
+ * with their scratch, run the kernels per patch (160, 192 in FP32) or the batched FFT kernels
+ * with a fused column stage.  Environment, read at plan creation: JUBIK_PLAN_MEMORY_MB bounds
+ * the device memory of one plan (10^6 bytes, fractions allowed); JUBIK_SEPARABLE=0 leaves the
+ * separable kernels out (debugging). */
 enum jubik_path {
   JUBIK_PATH_AUTO = 0,  /* fused when the FFT side and dtype allow it */
   JUBIK_PATH_FUSED = 1, /* FFT sides up to 128, and 160 and 192 in FP32.  160 and 192 run
                            the separable row and column kernels; the sides below one
                            kernel per patch unit: FFT, PSF product, overlap-add */
   JUBIK_PATH_PLAIN = 2, /* FFT sides 160, 192, 256, 320, 384 and 512 run the separable
-                           kernels in either precision; other sides, and plans whose
-                           separable scratch does not fit, batched FFT kernels + gather
-                           kernels.  The latter's per-module buffer is cut into module
+                           kernels in either precision; other sides batched FFT kernels +
+                           gather kernels, whose per-module buffer is cut into module
                            chunks of at most ~2 GiB; the environment variable
                            JUBIK_PLAIN_CHUNK_MODULES (a positive count, read at plan
                            creation) bounds the modules per chunk further.  Results do

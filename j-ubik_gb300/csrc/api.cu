@@ -230,6 +230,7 @@ struct jubik_plan {
   size_t esz = 4;
   int device = 0;
   size_t bytes = 0;
+  size_t bound = 0;  // device memory the plan may take (0: no bound)
   // constants
   void* wt = nullptr;  // (K) bilinear weights
   void* tw = nullptr;  // (P) fused twiddles
@@ -303,17 +304,15 @@ struct jubik_plan {
 
   int alloc(void** p, size_t n) {
     if (n == 0) n = 16;
+    if (bound && bytes + n > bound) {
+      set_error("plan workspace exceeds the %zu bytes that JUBIK_PLAN_MEMORY_MB allows", bound);
+      return JUBIK_ERR_ALLOC;
+    }
     cudaError_t e = cudaMalloc(p, n);
     if (e != cudaSuccess) return cuda_status(e, "cudaMalloc (plan workspace)");
     allocs.push_back(*p);
     bytes += n;
     return JUBIK_OK;
-  }
-  // frees the allocations made since `mark` (a size of allocs)
-  void release_from(size_t mark, size_t bytes_then) {
-    for (size_t i = mark; i < allocs.size(); ++i) cudaFree(allocs[i]);
-    allocs.resize(mark);
-    bytes = bytes_then;
   }
   ~jubik_plan() {
     for (int i = 0; i < JUBIK_PHASES; ++i) {
@@ -755,11 +754,143 @@ int sep_aligned(const jubik_plan* p, const void* out) {
   return JUBIK_OK;
 }
 
-// JUBIK_SEPARABLE=0 (read at plan creation, for debugging): plans take the kernels they
-// would take where the separable ones do not cover their field.
+// Environment read at plan creation: JUBIK_PLAN_MEMORY_MB, a bound of the device memory one
+// plan takes (MB of 10^6 bytes, fractions allowed); JUBIK_SEPARABLE=0, for debugging, leaves
+// the separable kernels out.
+size_t memory_bound() {
+  const char* env = std::getenv("JUBIK_PLAN_MEMORY_MB");
+  const double mb = env ? std::strtod(env, nullptr) : 0.0;
+  return mb > 0.0 && mb < 1e12 ? (size_t)(mb * 1e6) : 0;
+}
 bool separable_wanted() {
   const char* env = std::getenv("JUBIK_SEPARABLE");
   return !(env && env[0] == '0' && env[1] == 0);
+}
+
+// Makes the plan of a checked description, on the separable kernels (sep) or without them.
+// JUBIK_ERR_ALLOC where its device memory does not fit; nothing is kept then.
+int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubik_plan** out) {
+  // modules share the patch spectra (sky forward, summed adjoint) when there are several
+  const bool share = path == JUBIK_PATH_FUSED && d->path != JUBIK_PATH_FUSED_UNIT && g.M >= 2;
+  jubik_plan* p = new (std::nothrow) jubik_plan();
+  if (!p) {
+    set_error("host allocation failed");
+    return JUBIK_ERR_ALLOC;
+  }
+  p->desc = *d;
+  p->g = g;
+  p->dtype = d->dtype;
+  p->esz = d->dtype == JUBIK_F32 ? 4 : 8;
+  p->path = path;
+  p->bound = memory_bound();
+  cudaGetDevice(&p->device);
+  int st = JUBIK_OK;
+  auto fail = [&](int s) {
+    delete p;
+    return s;
+  };
+  const size_t csz = 2 * p->esz;
+  const int64_t units = g.units();
+  const int64_t img = (int64_t)g.M * g.E * g.pixels();
+  // constants
+  {
+    std::vector<double> b = bilinear_vector(g.K);
+    if ((st = p->alloc(&p->wt, g.K * p->esz))) return fail(st);
+    if (p->dtype == JUBIK_F32) {
+      std::vector<float> bf(b.begin(), b.end());
+      if ((st = cuda_status(cudaMemcpy(p->wt, bf.data(), g.K * 4, cudaMemcpyHostToDevice),
+                            "upload weights")))
+        return fail(st);
+    } else {
+      if ((st = cuda_status(cudaMemcpy(p->wt, b.data(), g.K * 8, cudaMemcpyHostToDevice),
+                            "upload weights")))
+        return fail(st);
+    }
+  }
+  if ((st = fft1d_init(&p->fft, g.P))) return fail(st);
+  p->tw = p->dtype == JUBIK_F32 ? p->fft.tw32 : p->fft.tw64;
+  if (sep) {
+    const SepSizes z = sep_sizes(g, d->dtype);
+    p->sep = true;
+    if ((st = upload_sep_tables(p))) return fail(st);
+    if ((st = p->alloc(&p->sky_rows, z.sky_rows))) return fail(st);
+    if ((st = p->alloc(&p->fwd_slabs, z.fwd_slabs))) return fail(st);
+    if ((st = p->alloc(&p->img_rows, z.img_rows))) return fail(st);
+    if ((st = p->alloc(&p->grad_slabs, z.grad_slabs))) return fail(st);
+  }
+  if (sep || p->path == JUBIK_PATH_FUSED) {
+    if ((st = p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz))) return fail(st);
+    if ((st = p->alloc(&p->hnyq, (size_t)units * g.P * csz))) return fail(st);
+  }
+  if (p->path == JUBIK_PATH_FUSED) {
+    if (share && (st = p->alloc(&p->spec, fused_spec_bytes(g, p->dtype)))) return fail(st);
+    if (share && (st = p->alloc(&p->acc, fused_spec_bytes(g, p->dtype)))) return fail(st);
+    if (share && (st = cuda_status(cudaMemset(p->acc, 0, fused_spec_bytes(g, p->dtype)),
+                                   "memset accumulator")))
+      return fail(st);
+    const int64_t patches = (int64_t)g.E * g.n * g.n;
+    if (share) {
+      p->adj_grid = fused_adj_grid(g, p->dtype);
+      if (p->adj_grid <= 0) {
+        delete p;
+        set_error("no launch configuration for the ordered adjoint at P=%d", g.P);
+        return JUBIK_ERR_UNSUPPORTED;
+      }
+      if ((st = p->alloc(&p->spill, (size_t)p->adj_grid * g.P * (g.P / 2) * csz)))
+        return fail(st);
+    }
+    if ((st = p->alloc(&p->conv_lo, img * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->conv_v_lo, img * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->grad_lo, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->bnd_f, sizeof(uint64_t) * std::max<int64_t>(patches,
+                                                                        kMaxBoundBlocks))))
+      return fail(st);
+    if ((st = p->alloc(&p->bnd_a, sizeof(uint64_t) *
+                                      std::max<int64_t>(energy_partials_count(), kMaxBoundBlocks))))
+      return fail(st);
+  } else if (!p->sep) {
+    if ((st = p->alloc(&p->hfull, (size_t)units * g.P * (g.P / 2 + 1) * csz))) return fail(st);
+    if ((st = p->alloc(&p->zs, (size_t)plain_pairs(g) * g.P * g.P * csz))) return fail(st);
+    // bound the per-chunk unit buffer to ~2 GiB; JUBIK_PLAIN_CHUNK_MODULES, when
+    // set to a positive count, bounds the modules per chunk further
+    const size_t per_module = (size_t)plain_pairs(g) * g.P * g.P * csz;
+    size_t chunk = std::min<size_t>(g.M, (2ull << 30) / per_module);
+    if (const char* env = std::getenv("JUBIK_PLAIN_CHUNK_MODULES")) {
+      const long v = std::strtol(env, nullptr, 10);
+      if (v >= 1) chunk = std::min<size_t>(chunk, (size_t)v);
+    }
+    p->zu_modules = (int)std::max<size_t>(1, chunk);
+    if ((st = p->alloc(&p->zu, per_module * p->zu_modules))) return fail(st);
+  }
+  if (!p->sep || p->path == JUBIK_PATH_FUSED) {  // (a separable plan never stores these images)
+    if ((st = p->alloc(&p->conv, img * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->conv_v, img * p->esz))) return fail(st);
+    if ((st = p->alloc(&p->resid, img * p->esz))) return fail(st);
+  }
+  if ((st = p->alloc(&p->wts, img * p->esz))) return fail(st);
+  if ((st = p->alloc(&p->xsky, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
+  if ((st = p->alloc(&p->xgrad, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
+  if ((st = p->alloc((void**)&p->ridx, img * sizeof(int32_t)))) return fail(st);
+  if ((st = p->alloc((void**)&p->rlist, img * sizeof(int64_t)))) return fail(st);
+  if ((st = p->alloc((void**)&p->partials,
+                     2 * std::max(energy_partials_count(), kSepMaxBlocks) * sizeof(double))))
+    return fail(st);
+  if ((st = p->alloc((void**)&p->counter, sizeof(unsigned int)))) return fail(st);
+  if ((st = cuda_status(cudaMemset(p->counter, 0, sizeof(unsigned int)), "memset counter")))
+    return fail(st);
+  if (img > 0x7fffffffLL) {
+    delete p;
+    set_error("more than 2^31 image pixels per plan");
+    return JUBIK_ERR_UNSUPPORTED;
+  }
+  // default: everything read out, unit exposure
+  k_iota<<<blocks_for(img), 256>>>(p->ridx, p->rlist, img);
+  if ((st = cuda_status(cudaGetLastError(), "k_iota"))) return fail(st);
+  if ((st = cuda_status(cudaDeviceSynchronize(), "plan set-up"))) return fail(st);
+  p->readout_sizes.assign(g.M, (int64_t)g.E * g.pixels());
+  p->readout_total = img;
+  *out = p;
+  return JUBIK_OK;
 }
 
 int need(bool ok, const char* what) {
@@ -829,147 +960,28 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
     set_error("FFT side P=%d unsupported", g.P);
     return JUBIK_ERR_UNSUPPORTED;
   }
-  jubik_plan* p = new (std::nothrow) jubik_plan();
-  if (!p) {
-    set_error("host allocation failed");
-    return JUBIK_ERR_ALLOC;
-  }
-  p->desc = *d;
-  p->g = g;
-  p->dtype = d->dtype;
-  p->esz = d->dtype == JUBIK_F32 ? 4 : 8;
-  cudaGetDevice(&p->device);
   const bool fused_ok = fused_supported(g.P, d->dtype);
   if (d->path == JUBIK_PATH_FUSED && !fused_ok) {
-    delete p;
     set_error("fused path does not cover P=%d in this dtype", g.P);
     return JUBIK_ERR_UNSUPPORTED;
   }
   if (d->path < JUBIK_PATH_AUTO || d->path > JUBIK_PATH_FUSED_UNIT) {
-    delete p;
     set_error("unknown path %d", d->path);
     return JUBIK_ERR_INVALID_ARGUMENT;
   }
   if (d->path == JUBIK_PATH_FUSED_UNIT && !fused_ok) {
-    delete p;
     set_error("fused path does not cover P=%d in this dtype", g.P);
     return JUBIK_ERR_UNSUPPORTED;
   }
-  p->path = (d->path == JUBIK_PATH_PLAIN || !fused_ok) ? JUBIK_PATH_PLAIN : JUBIK_PATH_FUSED;
-  // modules share the patch spectra (sky forward, summed adjoint) when there are several
-  const bool share = p->path == JUBIK_PATH_FUSED && d->path != JUBIK_PATH_FUSED_UNIT && g.M >= 2;
-
-  int st = JUBIK_OK;
-  auto fail = [&](int s) {
-    delete p;
-    return s;
-  };
-  const size_t csz = 2 * p->esz;
-  const int64_t units = g.units();
-  const int64_t img = (int64_t)g.M * g.E * g.pixels();
-  // constants
-  {
-    std::vector<double> b = bilinear_vector(g.K);
-    if ((st = p->alloc(&p->wt, g.K * p->esz))) return fail(st);
-    if (p->dtype == JUBIK_F32) {
-      std::vector<float> bf(b.begin(), b.end());
-      if ((st = cuda_status(cudaMemcpy(p->wt, bf.data(), g.K * 4, cudaMemcpyHostToDevice),
-                            "upload weights")))
-        return fail(st);
-    } else {
-      if ((st = cuda_status(cudaMemcpy(p->wt, b.data(), g.K * 8, cudaMemcpyHostToDevice),
-                            "upload weights")))
-        return fail(st);
-    }
-  }
-  if ((st = fft1d_init(&p->fft, g.P))) return fail(st);
-  p->tw = p->dtype == JUBIK_F32 ? p->fft.tw32 : p->fft.tw64;
-  // the separable kernels where they cover the FFT side and their scratch fits
+  const int path = (d->path == JUBIK_PATH_PLAIN || !fused_ok) ? JUBIK_PATH_PLAIN : JUBIK_PATH_FUSED;
+  // the separable kernels where they cover the geometry and all of the plan fits with
+  // their scratch; else the kernels that take less
   if (d->path != JUBIK_PATH_FUSED_UNIT && separable_wanted() && sep_supported(g, d->dtype)) {
-    const SepSizes z = sep_sizes(g, d->dtype);
-    const size_t mark = p->allocs.size(), bytes = p->bytes;
-    p->sep = !upload_sep_tables(p) && !p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz) &&
-             !p->alloc(&p->hnyq, (size_t)units * g.P * csz) &&
-             !p->alloc(&p->sky_rows, z.sky_rows) && !p->alloc(&p->fwd_slabs, z.fwd_slabs) &&
-             !p->alloc(&p->img_rows, z.img_rows) && !p->alloc(&p->grad_slabs, z.grad_slabs);
-    if (!p->sep) {  // not enough memory: the paths with less scratch
-      cudaGetLastError();
-      p->release_from(mark, bytes);
-      p->hmain = p->hnyq = nullptr;
-      p->gains = nullptr;
-    }
+    const int st = build_plan(d, g, path, true, out);
+    if (st != JUBIK_ERR_ALLOC) return st;
+    cudaGetLastError();
   }
-  if (p->path == JUBIK_PATH_FUSED) {
-    if (!p->sep && (st = p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz))) return fail(st);
-    if (!p->sep && (st = p->alloc(&p->hnyq, (size_t)units * g.P * csz))) return fail(st);
-    if (share && (st = p->alloc(&p->spec, fused_spec_bytes(g, p->dtype)))) return fail(st);
-    if (share && (st = p->alloc(&p->acc, fused_spec_bytes(g, p->dtype)))) return fail(st);
-    if (share && (st = cuda_status(cudaMemset(p->acc, 0, fused_spec_bytes(g, p->dtype)),
-                                   "memset accumulator")))
-      return fail(st);
-    const int64_t patches = (int64_t)g.E * g.n * g.n;
-    if (share) {
-      p->adj_grid = fused_adj_grid(g, p->dtype);
-      if (p->adj_grid <= 0) {
-        delete p;
-        set_error("no launch configuration for the ordered adjoint at P=%d", g.P);
-        return JUBIK_ERR_UNSUPPORTED;
-      }
-      if ((st = p->alloc(&p->spill, (size_t)p->adj_grid * g.P * (g.P / 2) * csz)))
-        return fail(st);
-    }
-    if ((st = p->alloc(&p->conv_lo, img * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->conv_v_lo, img * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->grad_lo, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->bnd_f, sizeof(uint64_t) * std::max<int64_t>(patches,
-                                                                        kMaxBoundBlocks))))
-      return fail(st);
-    if ((st = p->alloc(&p->bnd_a, sizeof(uint64_t) *
-                                      std::max<int64_t>(energy_partials_count(), kMaxBoundBlocks))))
-      return fail(st);
-  } else if (!p->sep) {
-    if ((st = p->alloc(&p->hfull, (size_t)units * g.P * (g.P / 2 + 1) * csz))) return fail(st);
-    if ((st = p->alloc(&p->zs, (size_t)plain_pairs(g) * g.P * g.P * csz))) return fail(st);
-    // bound the per-chunk unit buffer to ~2 GiB; JUBIK_PLAIN_CHUNK_MODULES, when
-    // set to a positive count, bounds the modules per chunk further
-    const size_t per_module = (size_t)plain_pairs(g) * g.P * g.P * csz;
-    size_t chunk = std::min<size_t>(g.M, (2ull << 30) / per_module);
-    if (const char* env = std::getenv("JUBIK_PLAIN_CHUNK_MODULES")) {
-      const long v = std::strtol(env, nullptr, 10);
-      if (v >= 1) chunk = std::min<size_t>(chunk, (size_t)v);
-    }
-    p->zu_modules = (int)std::max<size_t>(1, chunk);
-    if ((st = p->alloc(&p->zu, per_module * p->zu_modules))) return fail(st);
-  }
-  if (!p->sep || p->path == JUBIK_PATH_FUSED) {  // (a separable plan never stores these images)
-    if ((st = p->alloc(&p->conv, img * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->conv_v, img * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->resid, img * p->esz))) return fail(st);
-  }
-  if ((st = p->alloc(&p->wts, img * p->esz))) return fail(st);
-  if ((st = p->alloc(&p->xsky, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
-  if ((st = p->alloc(&p->xgrad, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
-  if ((st = p->alloc((void**)&p->ridx, img * sizeof(int32_t)))) return fail(st);
-  if ((st = p->alloc((void**)&p->rlist, img * sizeof(int64_t)))) return fail(st);
-  if ((st = p->alloc((void**)&p->partials,
-                     2 * std::max(energy_partials_count(), kSepMaxBlocks) * sizeof(double))))
-    return fail(st);
-  if ((st = p->alloc((void**)&p->counter, sizeof(unsigned int)))) return fail(st);
-  if ((st = cuda_status(cudaMemset(p->counter, 0, sizeof(unsigned int)), "memset counter")))
-    return fail(st);
-  if (img > 0x7fffffffLL) {
-    delete p;
-    set_error("more than 2^31 image pixels per plan");
-    return JUBIK_ERR_UNSUPPORTED;
-  }
-  // default: everything read out, unit exposure
-  k_iota<<<blocks_for(img), 256>>>(p->ridx, p->rlist, img);
-  if ((st = cuda_status(cudaGetLastError(), "k_iota"))) return fail(st);
-  if ((st = cuda_status(cudaDeviceSynchronize(), "plan set-up"))) return fail(st);
-  p->readout_sizes.assign(g.M, (int64_t)g.E * g.pixels());
-  p->readout_total = img;
-  *out = p;
-  return JUBIK_OK;
+  return build_plan(d, g, path, false, out);
 }
 
 int jubik_plan_destroy(jubik_plan* plan) {
