@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -279,15 +280,21 @@ struct jubik_plan {
   void* zu = nullptr;
   int zu_modules = 0;
   // separable path (sep.h): the entry points of this plan run its row and column
-  // kernels; a fused plan's other buffers then serve grouped launches only
+  // kernels; the fused kernels' buffers come with the first group a fused plan joins
   bool sep = false;
+  bool shared = false;   // fused path: modules share the patch spectra
+  std::mutex grouped;    // guards the buffers of grouped launches on a separable plan
   void* ramp = nullptr;  // (K) window weights times (dx - 1) / 2^ramp_log2, exact
   int ramp_log2 = 0;
   double* gains = nullptr;  // (2, P) gains less one of the column and row transforms (FP32)
+  // Two buffers serve four arrays: when the image rows are written the sky rows have been
+  // read, and the forward slabs when the gradient slabs are (each kernel waits for the one
+  // before it, and the writers follow the last readers).
   void* sky_rows = nullptr;
-  void* fwd_slabs = nullptr;
   void* img_rows = nullptr;
+  void* fwd_slabs = nullptr;
   void* grad_slabs = nullptr;
+  size_t slab_bytes = 0;  // of fwd_slabs
   // state
   bool psf_set = false, exposure_set = false, data_set = false, lam_valid = false;
   // bumped whenever a buffer address or the readout map that a group copied in
@@ -313,6 +320,12 @@ struct jubik_plan {
     allocs.push_back(*p);
     bytes += n;
     return JUBIK_OK;
+  }
+  // frees the allocations made since `mark` (a size of allocs)
+  void release_from(size_t mark, size_t bytes_then) {
+    for (size_t i = mark; i < allocs.size(); ++i) cudaFree(allocs[i]);
+    allocs.resize(mark);
+    bytes = bytes_then;
   }
   ~jubik_plan() {
     for (int i = 0; i < JUBIK_PHASES; ++i) {
@@ -633,7 +646,7 @@ int upload_sep_tables(jubik_plan* p) {
 
 // Run length is a setting of this plan (module-shared FP32 kernels at FFT side 192).
 bool sets_forward_run(const jubik_plan* p) {
-  return p->path == JUBIK_PATH_FUSED && p->spec && p->dtype == JUBIK_F32 && p->g.P == 192;
+  return p->path == JUBIK_PATH_FUSED && p->shared && p->dtype == JUBIK_F32 && p->g.P == 192;
 }
 // Patches per run of the forward's columns: the setting, or the library's choice.
 int forward_run_of(const jubik_plan* p) {
@@ -767,11 +780,60 @@ bool separable_wanted() {
   return !(env && env[0] == '0' && env[1] == 0);
 }
 
+// Buffers of the fused kernels: those of grouped launches, and (alone) those that only the
+// plan's own calls use.
+int alloc_grouped(jubik_plan* p) {
+  const Geom& g = p->g;
+  const int64_t img = (int64_t)g.M * g.E * g.pixels();
+  if (p->shared) {
+    const size_t bytes = fused_spec_bytes(g, p->dtype);
+    JUBIK_TRY(p->alloc(&p->spec, bytes));
+    JUBIK_TRY(p->alloc(&p->acc, bytes));
+    JUBIK_TRY_CUDA(cudaMemset(p->acc, 0, bytes));
+    p->adj_grid = fused_adj_grid(g, p->dtype);
+    if (p->adj_grid <= 0) {
+      set_error("no launch configuration for the ordered adjoint at P=%d", g.P);
+      return JUBIK_ERR_UNSUPPORTED;
+    }
+    JUBIK_TRY(p->alloc(&p->spill, (size_t)p->adj_grid * g.P * (g.P / 2) * 2 * p->esz));
+  }
+  JUBIK_TRY(p->alloc(&p->conv_lo, img * p->esz));
+  JUBIK_TRY(p->alloc(&p->grad_lo, (size_t)g.E * g.pixels() * p->esz));
+  JUBIK_TRY(p->alloc(&p->bnd_a, sizeof(uint64_t) * std::max<int64_t>(energy_partials_count(),
+                                                                     kMaxBoundBlocks)));
+  JUBIK_TRY(p->alloc(&p->conv, img * p->esz));
+  return p->alloc(&p->resid, img * p->esz);
+}
+int alloc_fused(jubik_plan* p) {
+  const Geom& g = p->g;
+  const int64_t img = (int64_t)g.M * g.E * g.pixels();
+  JUBIK_TRY(alloc_grouped(p));
+  JUBIK_TRY(p->alloc(&p->conv_v, img * p->esz));
+  JUBIK_TRY(p->alloc(&p->conv_v_lo, img * p->esz));
+  return p->alloc(&p->bnd_f, sizeof(uint64_t) * std::max<int64_t>((int64_t)g.E * g.n * g.n,
+                                                                  kMaxBoundBlocks));
+}
+
+// The buffers of grouped launches on a separable plan, made when it first joins a group.
+int join_group(jubik_plan* p) {
+  if (!p->sep) return JUBIK_OK;
+  std::lock_guard<std::mutex> lock(p->grouped);
+  if (p->resid) return JUBIK_OK;  // (the last of them)
+  const size_t mark = p->allocs.size(), bytes = p->bytes;
+  int st = alloc_grouped(p);
+  if (!st) st = cuda_status(cudaStreamSynchronize(nullptr), "group buffers");
+  if (st) {
+    p->release_from(mark, bytes);
+    p->spec = p->acc = p->spill = p->conv_lo = p->grad_lo = p->conv = p->resid = nullptr;
+    p->bnd_a = nullptr;
+    cudaGetLastError();
+  }
+  return st;
+}
+
 // Makes the plan of a checked description, on the separable kernels (sep) or without them.
 // JUBIK_ERR_ALLOC where its device memory does not fit; nothing is kept then.
 int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubik_plan** out) {
-  // modules share the patch spectra (sky forward, summed adjoint) when there are several
-  const bool share = path == JUBIK_PATH_FUSED && d->path != JUBIK_PATH_FUSED_UNIT && g.M >= 2;
   jubik_plan* p = new (std::nothrow) jubik_plan();
   if (!p) {
     set_error("host allocation failed");
@@ -782,6 +844,8 @@ int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubi
   p->dtype = d->dtype;
   p->esz = d->dtype == JUBIK_F32 ? 4 : 8;
   p->path = path;
+  // modules share the patch spectra (sky forward, summed adjoint) when there are several
+  p->shared = path == JUBIK_PATH_FUSED && d->path != JUBIK_PATH_FUSED_UNIT && g.M >= 2;
   p->bound = memory_bound();
   cudaGetDevice(&p->device);
   int st = JUBIK_OK;
@@ -810,44 +874,21 @@ int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubi
   if ((st = fft1d_init(&p->fft, g.P))) return fail(st);
   p->tw = p->dtype == JUBIK_F32 ? p->fft.tw32 : p->fft.tw64;
   if (sep) {
-    const SepSizes z = sep_sizes(g, d->dtype);
+    const SepSizes z = sep_sizes(g, d->dtype, sep_auto_run(g, d->dtype));
     p->sep = true;
     if ((st = upload_sep_tables(p))) return fail(st);
-    if ((st = p->alloc(&p->sky_rows, z.sky_rows))) return fail(st);
-    if ((st = p->alloc(&p->fwd_slabs, z.fwd_slabs))) return fail(st);
+    p->slab_bytes = std::max(z.fwd_slabs, z.grad_slabs);
+    if ((st = p->alloc(&p->fwd_slabs, p->slab_bytes))) return fail(st);
     if ((st = p->alloc(&p->img_rows, z.img_rows))) return fail(st);
-    if ((st = p->alloc(&p->grad_slabs, z.grad_slabs))) return fail(st);
+    p->grad_slabs = p->fwd_slabs;
+    p->sky_rows = p->img_rows;  // (one module's rows, M of them there)
   }
   if (sep || p->path == JUBIK_PATH_FUSED) {
     if ((st = p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz))) return fail(st);
     if ((st = p->alloc(&p->hnyq, (size_t)units * g.P * csz))) return fail(st);
   }
   if (p->path == JUBIK_PATH_FUSED) {
-    if (share && (st = p->alloc(&p->spec, fused_spec_bytes(g, p->dtype)))) return fail(st);
-    if (share && (st = p->alloc(&p->acc, fused_spec_bytes(g, p->dtype)))) return fail(st);
-    if (share && (st = cuda_status(cudaMemset(p->acc, 0, fused_spec_bytes(g, p->dtype)),
-                                   "memset accumulator")))
-      return fail(st);
-    const int64_t patches = (int64_t)g.E * g.n * g.n;
-    if (share) {
-      p->adj_grid = fused_adj_grid(g, p->dtype);
-      if (p->adj_grid <= 0) {
-        delete p;
-        set_error("no launch configuration for the ordered adjoint at P=%d", g.P);
-        return JUBIK_ERR_UNSUPPORTED;
-      }
-      if ((st = p->alloc(&p->spill, (size_t)p->adj_grid * g.P * (g.P / 2) * csz)))
-        return fail(st);
-    }
-    if ((st = p->alloc(&p->conv_lo, img * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->conv_v_lo, img * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->grad_lo, (size_t)g.E * g.pixels() * p->esz))) return fail(st);
-    if ((st = p->alloc(&p->bnd_f, sizeof(uint64_t) * std::max<int64_t>(patches,
-                                                                        kMaxBoundBlocks))))
-      return fail(st);
-    if ((st = p->alloc(&p->bnd_a, sizeof(uint64_t) *
-                                      std::max<int64_t>(energy_partials_count(), kMaxBoundBlocks))))
-      return fail(st);
+    if (!sep && (st = alloc_fused(p))) return fail(st);
   } else if (!p->sep) {
     if ((st = p->alloc(&p->hfull, (size_t)units * g.P * (g.P / 2 + 1) * csz))) return fail(st);
     if ((st = p->alloc(&p->zs, (size_t)plain_pairs(g) * g.P * g.P * csz))) return fail(st);
@@ -862,7 +903,7 @@ int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubi
     p->zu_modules = (int)std::max<size_t>(1, chunk);
     if ((st = p->alloc(&p->zu, per_module * p->zu_modules))) return fail(st);
   }
-  if (!p->sep || p->path == JUBIK_PATH_FUSED) {  // (a separable plan never stores these images)
+  if (!sep && p->path == JUBIK_PATH_PLAIN) {  // (a separable plan never stores these images)
     if ((st = p->alloc(&p->conv, img * p->esz))) return fail(st);
     if ((st = p->alloc(&p->conv_v, img * p->esz))) return fail(st);
     if ((st = p->alloc(&p->resid, img * p->esz))) return fail(st);
@@ -1020,6 +1061,16 @@ int jubik_plan_set_forward_run(jubik_plan* p, int32_t run_len) {
     set_error("set_forward_run: runs of %d patches need the module-shared FP32 kernels at FFT "
               "side 192 with 64-pixel strides, a 32-pixel margin and %d | n", run_len, run_len);
     return JUBIK_ERR_UNSUPPORTED;
+  }
+  if (p->sep && run_len) {  // shorter runs leave more rows
+    const size_t need = sep_sizes(p->g, p->dtype, run_len).fwd_slabs;
+    if (need > p->slab_bytes) {
+      // (the former buffer stays: captured graphs may hold it)
+      void* slabs = nullptr;
+      JUBIK_TRY(p->alloc(&slabs, need));
+      p->fwd_slabs = slabs;
+      p->slab_bytes = need;
+    }
   }
   p->fwd_run = run_len;
   return JUBIK_OK;
@@ -1663,6 +1714,8 @@ int jubik_group_create(jubik_plan* const* plans, int32_t n, jubik_group** out) {
     } else if (!p->psf_set || !p->data_set) {
       set_error("group: plan %d needs its PSF and data set", i);
       st = JUBIK_ERR_STATE;
+    } else {
+      st = join_group(p);
     }
     if (st) {
       delete g;
@@ -1673,7 +1726,7 @@ int jubik_group_create(jubik_plan* const* plans, int32_t n, jubik_group** out) {
   g->dtype = plans[0]->dtype;
   for (int i = 0; i < n; ++i) {
     const int P = g->plans[i]->g.P;
-    const bool shared = g->plans[i]->spec != nullptr;
+    const bool shared = g->plans[i]->shared;
     auto it = std::find_if(g->classes.begin(), g->classes.end(), [&](const GroupClass& c) {
       return c.P == P && c.shared == shared;
     });

@@ -17,12 +17,12 @@ bool sep_supported(const Geom& g, int dtype) {
   return dtype == JUBIK_F32 ? sep_rows_fit<float>(g) : sep_rows_fit<double>(g);
 }
 
-SepSizes sep_sizes(const Geom& g, int dtype) {
+SepSizes sep_sizes(const Geom& g, int dtype, int run) {
   const size_t c = dtype == JUBIK_F32 ? 8 : 16, H = (size_t)g.P / 2;
   const size_t en2 = (size_t)g.E * g.n * g.n;
   SepSizes z;
   z.sky_rows = c * (size_t)g.E * g.n * g.nx * H;
-  z.fwd_slabs = c * (size_t)g.M * en2 * g.P * H;  // one patch per slab; longer runs take less
+  z.fwd_slabs = c * (size_t)g.M * g.E * g.n * (g.n / run) * ((run - 1) * g.dx + g.P) * H;
   z.img_rows = c * (size_t)g.M * g.E * g.n * g.nx * H;
   z.grad_slabs = c * en2 * g.K * H;
   return z;

@@ -74,12 +74,12 @@ struct SepCols {
 // FFT sides the separable kernels cover, given their shared memory for this
 // field (rows of ny pixels).
 bool sep_supported(const Geom& g, int dtype);
-// Scratch of a plan, in bytes: sky row spectra, forward slabs, image row
+// Scratch of a plan, in bytes: sky row spectra, forward slabs of `run` patches, image row
 // spectra, gradient slabs.
 struct SepSizes {
   size_t sky_rows, fwd_slabs, img_rows, grad_slabs;
 };
-SepSizes sep_sizes(const Geom& g, int dtype);
+SepSizes sep_sizes(const Geom& g, int dtype, int run);
 // Gains less one of the column transforms (gy, by ky) and of the row transforms (gx, by kx)
 // of side P, each forward and back: P values each.
 void sep_gains(int P, std::vector<double>& gy, std::vector<double>& gx);

@@ -87,3 +87,43 @@ def test_memory_of_the_former_kernels_is_enough(cuda, name, monkeypatch):
     assert got[0] <= former[0] + 64
     tol = 2e-12 if prob.dtype == F64 else 2e-6
     assert np.linalg.norm(got[1] - full[1]) < tol * np.linalg.norm(full[1])
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_workspace(cuda, name, monkeypatch):
+    """The separable scratch takes two buffers, the slabs' and the rows'.  Against the former
+    kernels' workspace it weighs most with one module, which had no module-shared buffers:
+    4/3 of a spectrum per unit beside the spectrum itself, 1 + 4/3 over 1 + 5/9."""
+    prob = _Problem(name)
+    full = prob.run(monkeypatch)
+    monkeypatch.setenv("JUBIK_SEPARABLE", "0")
+    assert full[0] <= 1.5 * prob.run(monkeypatch)[0]
+
+
+def test_longer_slabs_keep_captured_graphs_valid(cuda):
+    """A shorter run takes larger slabs; a graph captured before goes on with its own."""
+    rng = np.random.default_rng(3)
+    nx, n = 256, 4
+    u = np.arange(128) - 64
+    psf = np.exp(-0.5 * (u[:, None] ** 2 + u[None, :] ** 2) / rng.uniform(
+        1.0, 4.0, size=(2, n * n, 1, 1, 1)) ** 2)
+    plan = ju.ResponsePlan(2, 1, (nx, nx), n, 32, dtype=F32)
+    try:
+        plan.set_psf(psf)
+        x = torch.as_tensor(np.exp(rng.normal(size=(1, nx, nx))), dtype=F32, device=cuda)
+        out = torch.empty((2, 1, nx, nx), dtype=F32, device=cuda)
+        want = {}
+        for r in (4, 1):
+            plan.set_forward_run(r)
+            want[r] = plan.psf_forward(x, out=out).clone()
+        plan.set_forward_run(4)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            plan.psf_forward(x, out=out)
+        plan.set_forward_run(1)
+        assert torch.equal(plan.psf_forward(x, out=out), want[1])
+        graph.replay()
+        assert torch.equal(out, want[4])
+    finally:
+        plan.close()
