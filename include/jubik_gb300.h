@@ -189,8 +189,7 @@ JUBIK_API int jubik_plan_set_dependent_launch(jubik_plan* plan, int32_t on);
  * across run lengths and are the same bits for a given one.  Returns
  * JUBIK_ERR_UNSUPPORTED for runs the plan's geometry cannot take. */
 JUBIK_API int jubik_plan_set_forward_run(jubik_plan* plan, int32_t run_len);
-/* The run length the plan's forward uses (1 where it is not a setting of the plan: other
- * FFT sides, FP64 and one-module plans, whose schedule the library always chooses). */
+/* The run length the plan's forward uses: the one set, or the library's choice. */
 JUBIK_API int jubik_plan_forward_run(const jubik_plan* plan, int32_t* run_len);
 JUBIK_API int jubik_plan_set_profiling(jubik_plan* plan, int32_t on);
 /* ms and launch counts per phase accumulated since profiling was switched on. */

@@ -652,8 +652,8 @@ bool sets_forward_run(const jubik_plan* p) {
 int forward_run_of(const jubik_plan* p) {
   if (!p->sep)
     return sets_forward_run(p) ? fused_fwd_run_len(p->g, p->dtype, p->fwd_run) : 1;
-  if (sets_forward_run(p) && p->fwd_run) return p->fwd_run;
-  return sep_auto_run(p->g, p->dtype);
+  // (longer runs than 1 are a setting of some plans only; see jubik_plan_set_forward_run)
+  return p->fwd_run ? p->fwd_run : sep_auto_run(p->g, p->dtype);
 }
 
 // The factor of a pass in two words: `scale`, and what the exact weights leave out of the
@@ -1082,7 +1082,7 @@ int jubik_plan_forward_run(const jubik_plan* p, int32_t* run_len) {
     set_error("forward_run: null output");
     return JUBIK_ERR_INVALID_ARGUMENT;
   }
-  *run_len = sets_forward_run(p) ? forward_run_of(p) : 1;
+  *run_len = forward_run_of(p);
   return JUBIK_OK;
 }
 

@@ -166,8 +166,7 @@ class ResponsePlan:
 
     @property
     def forward_run(self) -> int:
-        """The run length the forward uses (1 where it is not a setting of the plan:
-        other FFT sides, FP64 and one-module plans)."""
+        """The run length the forward uses: the one set, or the library's choice."""
         r = C.c_int32()
         _lib.call("jubik_plan_forward_run", self._h, C.byref(r))
         return int(r.value)
