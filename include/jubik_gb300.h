@@ -43,9 +43,10 @@ enum jubik_status {
 
 enum jubik_dtype { JUBIK_F32 = 0, JUBIK_F64 = 1 };
 
-/* Fields too wide for the separable row kernels, and plans that do not fit in device memory
- * with their scratch, run the kernels per patch (160, 192 in FP32) or the batched FFT kernels
- * with a fused column stage.  Environment, read at plan creation: JUBIK_PLAN_MEMORY_MB bounds
+/* Plans that do not fit in device memory with the separable scratch take one module at a time
+ * (the same bits).  Those that still do not fit, and fields too wide for the separable row
+ * kernels, run the kernels per patch (160, 192 in FP32) or the batched FFT kernels with a
+ * fused column stage.  Environment, read at plan creation: JUBIK_PLAN_MEMORY_MB bounds
  * the device memory of one plan (10^6 bytes, fractions allowed); JUBIK_SEPARABLE=0 leaves the
  * separable kernels out (debugging). */
 enum jubik_path {
@@ -56,9 +57,9 @@ enum jubik_path {
   JUBIK_PATH_PLAIN = 2, /* FFT sides 160, 192, 256, 320, 384 and 512 run the separable
                            kernels in either precision; other sides batched FFT kernels +
                            gather kernels, whose per-module buffer is cut into module
-                           chunks of at most ~2 GiB; the environment variable
+                           chunks of at most ~2 GiB.  The environment variable
                            JUBIK_PLAIN_CHUNK_MODULES (a positive count, read at plan
-                           creation) bounds the modules per chunk further.  Results do
+                           creation) bounds the modules in flight on either.  Results do
                            not depend on the chunking. */
   JUBIK_PATH_FUSED_UNIT = 3 /* fused, one kernel per (module, energy, patch) unit with no
                                sharing of patch spectra across modules */

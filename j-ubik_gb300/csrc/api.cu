@@ -287,9 +287,12 @@ struct jubik_plan {
   void* ramp = nullptr;  // (K) window weights times (dx - 1) / 2^ramp_log2, exact
   int ramp_log2 = 0;
   double* gains = nullptr;  // (2, P) gains less one of the column and row transforms (FP32)
-  // Two buffers serve four arrays: when the image rows are written the sky rows have been
+  int sep_modules = 0;  // modules per chunk (all of them, unless memory is short)
+  void* sep_state = nullptr;  // several chunks: the likelihood's sums so far
+  // With one chunk, two buffers serve four arrays: when the image rows are written the sky rows have been
   // read, and the forward slabs when the gradient slabs are (each kernel waits for the one
-  // before it, and the writers follow the last readers).
+  // before it, and the writers follow the last readers).  The sky rows of several chunks
+  // have their own.
   void* sky_rows = nullptr;
   void* img_rows = nullptr;
   void* fwd_slabs = nullptr;
@@ -665,19 +668,64 @@ void sep_scale(const jubik_plan* p, double scale, SepRows* r) {
   r->scale_lo = std::fma(-r->scale, d, a) / d;
 }
 
-// Forward of the separable path: sky rows, columns, image rows handed to `mode`
-// (onward: and on to the row spectra of the rows the adjoint starts from).
-int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMode mode, void* out,
-                bool onward, double* energy, cudaStream_t s) {
-  const Geom& g = p->g;
-  SepCols c;
-  c.rows = p->sky_rows;
-  c.hmain = p->hmain;
-  c.hnyq = p->hnyq;
+// Modules [m0, m0 + nm) of a separable plan: geometry and arguments of their launches.
+struct SepChunk {
+  Geom g;
+  SepRows rows;  // of the image's planes
+  SepCols cols;
+};
+SepChunk sep_chunk_of(const jubik_plan* p, int m0) {
+  SepChunk k;
+  k.g = p->g;
+  k.g.M = std::min(p->sep_modules, p->g.M - m0);
+  SepRows& r = k.rows;
+  r.tw = p->tw;
+  r.wt = p->ramp;
+  r.eps = p->eps;
+  r.dimg = p->dimg;
+  r.ridx = p->ridx;
+  r.wts = p->wts;
+  r.partials = p->partials;
+  r.counter = p->counter;
+  r.state = p->sep_state;
+  r.plane0 = m0 * p->g.E;
+  r.planes = k.g.M * p->g.E;
+  r.all_planes = p->g.M * p->g.E;
+  const int64_t spectra = (int64_t)m0 * p->g.n * p->g.n * p->g.E * p->g.P * 2 * p->esz;
+  SepCols& c = k.cols;
+  c.hmain = (const char*)p->hmain + spectra * (p->g.P / 2);
+  c.hnyq = (const char*)p->hnyq + spectra;
   c.tw = p->tw;
   c.wt = p->ramp;
-  c.slab = p->fwd_slabs;
   c.run = forward_run_of(p);
+  return k;
+}
+
+// Adjoint columns of a chunk, from the row spectra in img_rows.
+int sep_adjoint_cols(jubik_plan* p, SepChunk& k, int m0, cudaStream_t s) {
+  Phase ph(p, 1, s);
+  k.cols.rows = p->img_rows;
+  k.cols.slab = p->grad_slabs;
+  k.cols.run = (m0 > 0 ? SEP_RESUME : 0) | (m0 + k.g.M < p->g.M ? SEP_PASS_ON : 0);
+  return sep_cols(k.g, p->dtype, SEP_COLS_ADJ, k.cols, p->pdl, s);
+}
+int sep_gradient_rows(jubik_plan* p, void* out_x, double scale, cudaStream_t s) {
+  Phase ph(p, 5, s);
+  SepRows r;
+  r.slab = p->grad_slabs;
+  r.out = out_x;
+  r.tw = p->tw;
+  r.wt = p->ramp;
+  sep_scale(p, scale, &r);
+  r.planes = p->g.E;
+  return sep_rows(p->g, p->dtype, SEP_GRAD, r, p->pdl, s);
+}
+
+// Forward of the separable path: sky rows, then per module chunk the columns and the image
+// rows, handed to `mode`; with grad_x, on to the rows the adjoint starts from, and the adjoint.
+int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMode mode, void* out,
+                void* grad_x, double* energy, cudaStream_t s) {
+  const Geom& g = p->g;
   {
     Phase ph(p, 4, s);
     SepRows r;
@@ -691,71 +739,43 @@ int sep_forward(jubik_plan* p, const void* x, SkyView view, double scale, SepMod
     r.planes = g.E;
     JUBIK_TRY(sep_rows(g, p->dtype, SEP_SKY, r, p->pdl, s));
   }
-  {
-    Phase ph(p, 0, s);
-    JUBIK_TRY(sep_cols(g, p->dtype, SEP_COLS_FWD, c, p->pdl, s));
+  for (int m0 = 0; m0 < g.M; m0 += p->sep_modules) {
+    SepChunk k = sep_chunk_of(p, m0);
+    {
+      Phase ph(p, 0, s);
+      k.cols.rows = p->sky_rows;
+      k.cols.slab = p->fwd_slabs;
+      JUBIK_TRY(sep_cols(k.g, p->dtype, SEP_COLS_FWD, k.cols, p->pdl, s));
+    }
+    {
+      Phase ph(p, 2, s);
+      k.rows.slab = p->fwd_slabs;
+      k.rows.slab_run = k.cols.run;
+      k.rows.rows = grad_x ? p->img_rows : nullptr;
+      k.rows.out = out;
+      k.rows.energy = energy;
+      sep_scale(p, scale, &k.rows);
+      JUBIK_TRY(sep_rows(k.g, p->dtype, mode, k.rows, p->pdl, s));
+    }
+    if (grad_x) JUBIK_TRY(sep_adjoint_cols(p, k, m0, s));
   }
-  Phase ph(p, 2, s);
-  SepRows r;
-  r.slab = p->fwd_slabs;
-  r.slab_run = c.run;
-  r.rows = onward ? p->img_rows : nullptr;
-  r.out = out;
-  r.tw = p->tw;
-  r.wt = p->ramp;
-  r.eps = p->eps;
-  r.dimg = p->dimg;
-  r.ridx = p->ridx;
-  r.wts = p->wts;
-  r.partials = p->partials;
-  r.counter = p->counter;
-  r.energy = energy;
-  sep_scale(p, scale, &r);
-  r.planes = g.M * g.E;
-  return sep_rows(g, p->dtype, mode, r, p->pdl, s);
-}
-
-// Adjoint of the separable path from the row spectra in img_rows.
-int sep_adjoint(jubik_plan* p, void* out_x, double scale, cudaStream_t s) {
-  const Geom& g = p->g;
-  {
-    Phase ph(p, 1, s);
-    SepCols c;
-    c.rows = p->img_rows;
-    c.hmain = p->hmain;
-    c.hnyq = p->hnyq;
-    c.tw = p->tw;
-    c.wt = p->ramp;
-    c.slab = p->grad_slabs;
-    JUBIK_TRY(sep_cols(g, p->dtype, SEP_COLS_ADJ, c, p->pdl, s));
-  }
-  Phase ph(p, 5, s);
-  SepRows r;
-  r.slab = p->grad_slabs;
-  r.out = out_x;
-  r.tw = p->tw;
-  r.wt = p->ramp;
-  sep_scale(p, scale, &r);
-  r.planes = g.E;
-  return sep_rows(g, p->dtype, SEP_GRAD, r, p->pdl, s);
+  return grad_x ? sep_gradient_rows(p, grad_x, scale, s) : JUBIK_OK;
 }
 
 // Adjoint of an (M, E, nx, ny) image (SEP_COT) or a readout vector (SEP_COT_READOUT).
 int sep_adjoint_of(jubik_plan* p, const void* cot, SepMode mode, void* out_x, double scale,
                    cudaStream_t s) {
-  {
-    Phase ph(p, 2, s);
-    SepRows r;
-    r.in = cot;
-    r.rows = p->img_rows;
-    r.tw = p->tw;
-    r.wt = p->ramp;
-    r.eps = p->eps;
-    r.ridx = p->ridx;
-    r.planes = p->g.M * p->g.E;
-    JUBIK_TRY(sep_rows(p->g, p->dtype, mode, r, p->pdl, s));
+  for (int m0 = 0; m0 < p->g.M; m0 += p->sep_modules) {
+    SepChunk k = sep_chunk_of(p, m0);
+    {
+      Phase ph(p, 2, s);
+      k.rows.in = cot;
+      k.rows.rows = p->img_rows;
+      JUBIK_TRY(sep_rows(k.g, p->dtype, mode, k.rows, p->pdl, s));
+    }
+    JUBIK_TRY(sep_adjoint_cols(p, k, m0, s));
   }
-  return sep_adjoint(p, out_x, scale, s);
+  return sep_gradient_rows(p, out_x, scale, s);
 }
 
 // Results of fused plans are 16-byte aligned on every path (as combine_words asks).
@@ -774,6 +794,12 @@ size_t memory_bound() {
   const char* env = std::getenv("JUBIK_PLAN_MEMORY_MB");
   const double mb = env ? std::strtod(env, nullptr) : 0.0;
   return mb > 0.0 && mb < 1e12 ? (size_t)(mb * 1e6) : 0;
+}
+// JUBIK_PLAIN_CHUNK_MODULES: most modules of a plan of the plain path that are in flight.
+int chunk_modules() {
+  const char* env = std::getenv("JUBIK_PLAIN_CHUNK_MODULES");
+  const long v = env ? std::strtol(env, nullptr, 10) : 0;
+  return v >= 1 ? (int)std::min<long>(v, 1 << 30) : 1 << 30;
 }
 bool separable_wanted() {
   const char* env = std::getenv("JUBIK_SEPARABLE");
@@ -831,9 +857,10 @@ int join_group(jubik_plan* p) {
   return st;
 }
 
-// Makes the plan of a checked description, on the separable kernels (sep) or without them.
+// Makes the plan of a checked description, on the separable kernels (in chunks of sep modules)
+// or without them (0).
 // JUBIK_ERR_ALLOC where its device memory does not fit; nothing is kept then.
-int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubik_plan** out) {
+int build_plan(const jubik_plan_desc* d, const Geom& g, int path, int sep, jubik_plan** out) {
   jubik_plan* p = new (std::nothrow) jubik_plan();
   if (!p) {
     set_error("host allocation failed");
@@ -874,14 +901,23 @@ int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubi
   if ((st = fft1d_init(&p->fft, g.P))) return fail(st);
   p->tw = p->dtype == JUBIK_F32 ? p->fft.tw32 : p->fft.tw64;
   if (sep) {
-    const SepSizes z = sep_sizes(g, d->dtype, sep_auto_run(g, d->dtype));
+    const SepSizes z = sep_sizes(g, d->dtype, sep_auto_run(g, d->dtype), sep);
     p->sep = true;
+    p->sep_modules = sep;
     if ((st = upload_sep_tables(p))) return fail(st);
     p->slab_bytes = std::max(z.fwd_slabs, z.grad_slabs);
-    if ((st = p->alloc(&p->fwd_slabs, p->slab_bytes))) return fail(st);
+    // several chunks: the adjoint's sums between them, right behind the gradient slabs
+    const size_t sums = sep < g.M ? z.acc : 0;
+    if ((st = p->alloc(&p->fwd_slabs, p->slab_bytes + sums))) return fail(st);
     if ((st = p->alloc(&p->img_rows, z.img_rows))) return fail(st);
-    p->grad_slabs = p->fwd_slabs;
-    p->sky_rows = p->img_rows;  // (one module's rows, M of them there)
+    p->grad_slabs = (char*)p->fwd_slabs + (p->slab_bytes - z.grad_slabs);
+    p->sky_rows = p->img_rows;  // (one module's rows, several there)
+    if (sep < g.M) {
+      if ((st = p->alloc(&p->sky_rows, z.sky_rows))) return fail(st);
+      size_t state = 0;
+      if ((st = sep_state_bytes(g, d->dtype, &state))) return fail(st);
+      if ((st = p->alloc(&p->sep_state, state))) return fail(st);
+    }
   }
   if (sep || p->path == JUBIK_PATH_FUSED) {
     if ((st = p->alloc(&p->hmain, (size_t)units * g.P * (g.P / 2) * csz))) return fail(st);
@@ -895,11 +931,8 @@ int build_plan(const jubik_plan_desc* d, const Geom& g, int path, bool sep, jubi
     // bound the per-chunk unit buffer to ~2 GiB; JUBIK_PLAIN_CHUNK_MODULES, when
     // set to a positive count, bounds the modules per chunk further
     const size_t per_module = (size_t)plain_pairs(g) * g.P * g.P * csz;
-    size_t chunk = std::min<size_t>(g.M, (2ull << 30) / per_module);
-    if (const char* env = std::getenv("JUBIK_PLAIN_CHUNK_MODULES")) {
-      const long v = std::strtol(env, nullptr, 10);
-      if (v >= 1) chunk = std::min<size_t>(chunk, (size_t)v);
-    }
+    const size_t chunk = std::min<size_t>(std::min(g.M, chunk_modules()),
+                                          (2ull << 30) / per_module);
     p->zu_modules = (int)std::max<size_t>(1, chunk);
     if ((st = p->alloc(&p->zu, per_module * p->zu_modules))) return fail(st);
   }
@@ -1015,14 +1048,18 @@ int jubik_plan_create(const jubik_plan_desc* d, jubik_plan** out) {
     return JUBIK_ERR_UNSUPPORTED;
   }
   const int path = (d->path == JUBIK_PATH_PLAIN || !fused_ok) ? JUBIK_PATH_PLAIN : JUBIK_PATH_FUSED;
-  // the separable kernels where they cover the geometry and all of the plan fits with
-  // their scratch; else the kernels that take less
+  // the separable kernels where they cover the geometry and all of the plan fits with their
+  // scratch, if need be one module at a time; else the kernels that take less
   if (d->path != JUBIK_PATH_FUSED_UNIT && separable_wanted() && sep_supported(g, d->dtype)) {
-    const int st = build_plan(d, g, path, true, out);
-    if (st != JUBIK_ERR_ALLOC) return st;
-    cudaGetLastError();
+    const int most = path == JUBIK_PATH_PLAIN ? std::min(g.M, chunk_modules()) : g.M;
+    for (const int modules : {most, 1}) {
+      const int st = build_plan(d, g, path, modules, out);
+      if (st != JUBIK_ERR_ALLOC) return st;
+      cudaGetLastError();
+      if (modules == 1) break;
+    }
   }
-  return build_plan(d, g, path, false, out);
+  return build_plan(d, g, path, 0, out);
 }
 
 int jubik_plan_destroy(jubik_plan* plan) {
@@ -1063,7 +1100,7 @@ int jubik_plan_set_forward_run(jubik_plan* p, int32_t run_len) {
     return JUBIK_ERR_UNSUPPORTED;
   }
   if (p->sep && run_len) {  // shorter runs leave more rows
-    const size_t need = sep_sizes(p->g, p->dtype, run_len).fwd_slabs;
+    const size_t need = sep_sizes(p->g, p->dtype, run_len, p->sep_modules).fwd_slabs;
     if (need > p->slab_bytes) {
       // (the former buffer stays: captured graphs may hold it)
       void* slabs = nullptr;
@@ -1286,7 +1323,7 @@ int jubik_psf_forward(jubik_plan* p, const void* x, void* out, void* stream) {
   cudaStream_t s = S(stream);
   if (p->sep) {
     JUBIK_TRY(sep_aligned(p, out));
-    return sep_forward(p, x, SkyView(), 1.0, SEP_IMAGE, out, false, nullptr, s);
+    return sep_forward(p, x, SkyView(), 1.0, SEP_IMAGE, out, nullptr, nullptr, s);
   }
   JUBIK_TRY(do_forward(p, x, out, p->conv_lo, 1.0, s));
   return finish_words(p, out, p->conv_lo, image_elems(p), s);
@@ -1311,7 +1348,7 @@ int jubik_response_forward(jubik_plan* p, const void* x, void* out_readout, void
   JUBIK_TRY(need(p->psf_set, "PSF"));
   cudaStream_t s = S(stream);
   if (p->sep)
-    return sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_READOUT, out_readout, false,
+    return sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_READOUT, out_readout, nullptr,
                        nullptr, s);
   JUBIK_TRY(do_forward(p, x, p->conv, p->conv_lo, p->desc.pixel_area, s));
   const void* lo = p->path == JUBIK_PATH_FUSED ? p->conv_lo : nullptr;
@@ -1359,10 +1396,10 @@ int jubik_poisson_energy_grad(jubik_plan* p, const void* x, double* energy, void
   cudaStream_t s = S(stream);
   if (p->sep) {
     if (grad_x) JUBIK_TRY(sep_aligned(p, grad_x));
-    JUBIK_TRY(sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_LIKE, nullptr,
-                          grad_x != nullptr, energy, s));
+    JUBIK_TRY(sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_LIKE, nullptr, grad_x, energy,
+                          s));
     p->lam_valid = true;
-    return grad_x ? sep_adjoint(p, grad_x, p->desc.pixel_area, s) : JUBIK_OK;
+    return JUBIK_OK;
   }
   bool grad_zeroed = false;
   JUBIK_TRY(do_forward(p, x, p->conv, p->conv_lo, p->desc.pixel_area, s, grad_x,
@@ -1408,10 +1445,9 @@ int jubik_poisson_energy_grad_logsky(jubik_plan* p, const void* s_log, int32_t e
   const void* glo = nullptr;
   if (p->sep) {
     JUBIK_TRY(sep_forward(p, s_log, view, p->desc.pixel_area, SEP_LIKE, nullptr,
-                          grad_s != nullptr, energy, s));
+                          grad_s ? p->xgrad : nullptr, energy, s));
     p->lam_valid = true;
     if (!grad_s) return JUBIK_OK;
-    JUBIK_TRY(sep_adjoint(p, p->xgrad, p->desc.pixel_area, s));
   } else {
   bool grad_zeroed = false;
   JUBIK_TRY(do_forward(p, s_log, p->conv, p->conv_lo, p->desc.pixel_area, s,
@@ -1459,14 +1495,12 @@ int jubik_metric_apply(jubik_plan* p, const void* x, const void* v, void* out, v
   if (p->sep) {
     JUBIK_TRY(sep_aligned(p, out));
     if (x) {
-      JUBIK_TRY(sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_WEIGHTS, nullptr, false,
+      JUBIK_TRY(sep_forward(p, x, SkyView(), p->desc.pixel_area, SEP_WEIGHTS, nullptr, nullptr,
                             nullptr, s));
       p->lam_valid = true;
     }
     JUBIK_TRY(need(p->lam_valid, "lambda (call with x or after poisson_energy_grad)"));
-    JUBIK_TRY(sep_forward(p, v, SkyView(), p->desc.pixel_area, SEP_METRIC, nullptr, true, nullptr,
-                          s));
-    return sep_adjoint(p, out, p->desc.pixel_area, s);
+    return sep_forward(p, v, SkyView(), p->desc.pixel_area, SEP_METRIC, nullptr, out, nullptr, s);
   }
   const bool two = p->path == JUBIK_PATH_FUSED;
   if (x) {  // weights eps^2 / lam of a new lam = R(x), as the likelihood pass leaves them

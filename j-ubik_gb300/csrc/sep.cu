@@ -17,15 +17,24 @@ bool sep_supported(const Geom& g, int dtype) {
   return dtype == JUBIK_F32 ? sep_rows_fit<float>(g) : sep_rows_fit<double>(g);
 }
 
-SepSizes sep_sizes(const Geom& g, int dtype, int run) {
+SepSizes sep_sizes(const Geom& g, int dtype, int run, int modules) {
   const size_t c = dtype == JUBIK_F32 ? 8 : 16, H = (size_t)g.P / 2;
   const size_t en2 = (size_t)g.E * g.n * g.n;
   SepSizes z;
   z.sky_rows = c * (size_t)g.E * g.n * g.nx * H;
-  z.fwd_slabs = c * (size_t)g.M * g.E * g.n * (g.n / run) * ((run - 1) * g.dx + g.P) * H;
-  z.img_rows = c * (size_t)g.M * g.E * g.n * g.nx * H;
+  z.fwd_slabs = c * (size_t)modules * g.E * g.n * (g.n / run) * ((run - 1) * g.dx + g.P) * H;
+  z.img_rows = c * (size_t)modules * g.E * g.n * g.nx * H;
   z.grad_slabs = c * en2 * g.K * H;
+  z.acc = c * en2 * g.P * H;
   return z;
+}
+
+int sep_state_bytes(const Geom& g, int dtype, size_t* bytes) {
+  int64_t threads = 0;
+  JUBIK_TRY(dtype == JUBIK_F32 ? sep_like_threads_t<float>(g, &threads)
+                               : sep_like_threads_t<double>(g, &threads));
+  *bytes = (size_t)threads * 4 * (dtype == JUBIK_F32 ? 8 : 16);
+  return JUBIK_OK;
 }
 
 // The transforms' constants are rounded to FP32, so a transform and its inverse return

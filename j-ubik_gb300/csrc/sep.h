@@ -58,9 +58,18 @@ struct SepRows {
   unsigned int* counter = nullptr;
   double* energy = nullptr;
   double scale = 1.0, scale_lo = 0.0;  // the factor's two words
-  int planes = 0;              // M E, or E for SEP_SKY and SEP_GRAD
+  // Planes of the images (M E, or E for SEP_SKY and SEP_GRAD), and the module chunk of them
+  // that this launch takes: `planes` from plane0.  Slabs and row spectra hold the chunk only.
+  int all_planes = 0, plane0 = 0, planes = 0;
+  // SEP_LIKE in several chunks: per thread the sums of the chunks before (sep_state_bytes).
+  // Every launch has the grid of the whole image, and a CTA the items that it would take
+  // there, so the energy has the same bits however the modules are cut.
+  void* state = nullptr;
 };
 
+// Adjoint columns of a module chunk: the sums of the chunks before are read (RESUME), and
+// passed on instead of going to the gradient slabs (PASS_ON).  They lie behind the slabs.
+enum { SEP_RESUME = 1 << 8, SEP_PASS_ON = 1 << 9 };
 struct SepCols {
   const void* rows = nullptr;  // row spectra read
   const void* hmain = nullptr;
@@ -68,18 +77,24 @@ struct SepCols {
   const void* tw = nullptr;
   const void* wt = nullptr;
   void* slab = nullptr;        // slabs written
-  int run = 1;                 // forward: patches per slab
+  // forward: patches per slab; adjoint of a module chunk: SEP_RESUME | SEP_PASS_ON.  (More
+  // arguments, even unused ones, made the adjoint spill: 249 -> 261 us at 1024^2 x 7 x 3.)
+  int run = 1;
 };
 
 // FFT sides the separable kernels cover, given their shared memory for this
 // field (rows of ny pixels).
 bool sep_supported(const Geom& g, int dtype);
 // Scratch of a plan, in bytes: sky row spectra, forward slabs of `run` patches, image row
-// spectra, gradient slabs.
+// spectra, gradient slabs; module sums between chunks.
 struct SepSizes {
   size_t sky_rows, fwd_slabs, img_rows, grad_slabs;
+  size_t acc;  // several chunks only
 };
-SepSizes sep_sizes(const Geom& g, int dtype, int run);
+// (of `modules` modules at once)
+SepSizes sep_sizes(const Geom& g, int dtype, int run, int modules);
+// Bytes of the likelihood's sums between chunks: four complex values a thread.
+int sep_state_bytes(const Geom& g, int dtype, size_t* bytes);
 // Gains less one of the column transforms (gy, by ky) and of the row transforms (gx, by kx)
 // of side P, each forward and back: P values each.
 void sep_gains(int P, std::vector<double>& gy, std::vector<double>& gx);
@@ -98,6 +113,8 @@ template <typename T>
 int sep_rows_t(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaStream_t s);
 template <typename T>
 bool sep_rows_fit(const Geom& g);
+template <typename T>
+int sep_like_threads_t(const Geom& g, int64_t* threads);
 template <typename T>
 int sep_cols_t(const Geom& g, SepColsKind kind, const SepCols& a, bool pdl, cudaStream_t s);
 

@@ -447,12 +447,20 @@ __device__ __forceinline__ void col_fetch_rows(cx<T>* tile, const cx<T>* src, in
   }
 }
 
+// class it of patch u's sums between chunks, behind the gradient slabs
+template <typename T, int L1>
+__device__ __forceinline__ cx<T>* col_sums(const ColK& k, int u, int it) {
+  constexpr int P = 16 * L1, H = P / 2;
+  return (cx<T>*)k.a.slab + (int64_t)k.E * k.n2 * k.K * H + ((int64_t)u * P + 16 * it) * H;
+}
+
 // Adjoint columns of one patch: per module the row spectra of the patch's rows
 // -> spectrum -> conjugate PSF product, summed over modules in registers in
 // module order; the sum's inverse columns, weighted by the window rows, to the
 // patch's gradient slab.  The next module's rows arrive by cp.async in the other
-// tile, its PSF spectrum in registers, while this module is transformed.
-template <typename T, int L1>
+// tile, its PSF spectrum in registers, while this module is transformed.  CHUNK: the modules
+// come in several launches, and the sums wait behind the gradient slabs between them.
+template <typename T, int L1, bool CHUNK>
 __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::SMEM, 128))
     k_sep_cols_adj(ColK k) {
   using C = ColT<T, L1>;
@@ -486,6 +494,11 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
   cx<T> acc[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) acc[q] = mkc<T>((T)0, (T)0);
+  if (CHUNK && (k.a.run & SEP_RESUME) && mid) {
+    const cx<T>* sums = col_sums<T, L1>(k, u, it) + col;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) acc[q] = sums[q * H];
+  }
   for (int m = 0; m < k.M; ++m) {
     cx<T>* buf = tile + ((m & 1) ? C::TILE : 0);
     col_copy_wait();
@@ -527,6 +540,14 @@ __global__ void __launch_bounds__(ColT<T, L1>::NT, col_ctas<T, L1>(ColT<T, L1>::
     }
   }
   sep_trigger();
+  if (CHUNK && (k.a.run & SEP_PASS_ON)) {  // more module chunks to come
+    if (mid) {
+      cx<T>* sums = col_sums<T, L1>(k, u, it) + col;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) sums[q * H] = acc[q];
+    }
+    return;
+  }
   cx<T>* buf = tile + ((k.M & 1) ? C::TILE : 0);
   if (mid) spectrum_to_tile<T, L1>(buf + mine, mytw, acc);
   __syncthreads();
@@ -587,7 +608,7 @@ int dispatch_cols(const Geom& g, SepColsKind kind, const SepCols& a, bool pdl, c
   k.margin = g.margin;
   k.sr_max = g.sr_max;
   k.K = g.K;
-  k.nq = g.n / std::max(1, a.run);
+  k.nq = kind == SEP_COLS_FWD ? g.n / a.run : g.n;
   const int64_t patches = (int64_t)g.E * k.n2;
   const int64_t grid = (a.run > 1 && kind == SEP_COLS_FWD ? (int64_t)g.E * g.n * k.nq : patches) *
                        C::NG;
@@ -600,9 +621,15 @@ int dispatch_cols(const Geom& g, SepColsKind kind, const SepCols& a, bool pdl, c
   k.div_q = mulhi_divisor(k.nq, grid + 1);
   dim3 gd((unsigned)grid);
   int per_sm = 1;
+  if (kind == SEP_COLS_ADJ && (a.run & (SEP_RESUME | SEP_PASS_ON))) {
+    static SepKernelCache cache;
+    auto kern = k_sep_cols_adj<T, L1, true>;
+    JUBIK_TRY(cache.prepare((const void*)kern, C::NT, C::SMEM, &per_sm));
+    return sep_launch(kern, gd, C::NT, C::SMEM, pdl, s, "k_sep_cols_adj (chunk)", k);
+  }
   if (kind == SEP_COLS_ADJ) {
     static SepKernelCache cache;
-    auto kern = k_sep_cols_adj<T, L1>;
+    auto kern = k_sep_cols_adj<T, L1, false>;
     JUBIK_TRY(cache.prepare((const void*)kern, C::NT, C::SMEM, &per_sm));
     return sep_launch(kern, gd, C::NT, C::SMEM, pdl, s, "k_sep_cols_adj", k);
   }

@@ -36,7 +36,9 @@ struct RowK {
   int seqs;                  // sequences (row pair x window) in shared memory at once
   int rp;                    // row pairs per item
   int per;                   // items per plane
-  int items;                 // items in all
+  int grid_items;            // items of the whole image
+  int item0, items;          // this launch's items: item0 .. items - 1
+  int base;                  // the multiple of the grid before item0
   uint32_t mul_dx, mul_step;  // floor(u / d) = high word of u mul (row_div)
   uint32_t div_per;
   float scale32[2];  // the factor's two words
@@ -261,8 +263,18 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
   const T scale = row_scale<T>(k, 0), scale_lo = row_scale<T>(k, 1);
   Kahan2<T> s_lam, s_dlog;
   const int nchunk = (n * k.rp + k.seqs - 1) / k.seqs;  // > 1 only when rp == 1
+  if (MODE == SEP_LIKE && a.state && a.plane0) {  // the sums of the chunks before
+    const cx<T>* st = (const cx<T>*)a.state + 4 * ((int64_t)blockIdx.x * NT + tid);
+    s_lam.s = st[0];
+    s_lam.nc = st[1];
+    s_dlog.s = st[2];
+    s_dlog.nc = st[3];
+  }
+  // the first item of this launch that is this CTA's in the whole image
+  int item = k.base + blockIdx.x;
+  if (item < k.item0) item += gridDim.x;
 
-  for (int item = blockIdx.x; item < k.items; item += gridDim.x) {
+  for (; item < k.items; item += gridDim.x) {
     const int pl = sep_div(item, k.per, k.div_per);
     const int t0 = (item - pl * k.per) * k.rp;  // first row pair
     if (INV) {
@@ -619,6 +631,14 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
     }
   }
   if (MODE == SEP_LIKE) {
+    if (a.state && a.plane0 + a.planes < a.all_planes) {  // more chunks to come
+      cx<T>* st = (cx<T>*)a.state + 4 * ((int64_t)blockIdx.x * NT + tid);
+      st[0] = s_lam.s;
+      st[1] = s_lam.nc;
+      st[2] = s_dlog.s;
+      st[3] = s_dlog.nc;
+      return;
+    }
     __syncthreads();
     double* red = reinterpret_cast<double*>(smem_raw);  // every sequence has been read
     block_reduce2_of(s_lam.value(), s_dlog.value(), red, red + NT, a.partials, a.counter,
@@ -629,23 +649,34 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
 // bound of the numerators that the kernels divide by dx or a slab's stride
 inline int64_t sep_reach(const Geom& g) { return std::max(g.nx, g.ny) + 4 * (int64_t)g.P; }
 
+// Threads of a row CTA, and the grid: as many CTAs as fit at once, looping over the items
+// (the tables are built once per CTA, and the likelihood has one partial sum per CTA).
+inline int row_threads(const RowK& k) {
+  return 32 * ((std::min(k.seqs, k.n * k.rp) + 1) / 2);
+}
 template <typename T, int L1, int MODE, bool FWD>
-int launch_rows(const RowK& k, size_t smem, bool pdl, cudaStream_t s) {
-  auto kern = k_sep_rows<T, L1, MODE, FWD>;
-  int per_sm = 1;
+int row_grid(const RowK& k, size_t smem, int64_t* grid) {
   static SepKernelCache cache;
-  const int threads = 32 * ((std::min(k.seqs, k.n * k.rp) + 1) / 2);
-  JUBIK_TRY(cache.prepare((const void*)kern, threads, smem, &per_sm));
-  // as many CTAs as fit at once, looping over the items: the tables are built once per
-  // CTA, and the likelihood has one partial sum per CTA
-  const int64_t grid = std::min<int64_t>(
-      k.items, std::min<int64_t>(kSepMaxBlocks, (int64_t)sm_count() * per_sm));
-  return sep_launch(kern, dim3((unsigned)grid), threads, smem, pdl, s, "k_sep_rows", k);
+  int per_sm = 1;
+  JUBIK_TRY(cache.prepare((const void*)k_sep_rows<T, L1, MODE, FWD>, row_threads(k), smem,
+                          &per_sm));
+  *grid = std::min<int64_t>(k.grid_items,
+                            std::min<int64_t>(kSepMaxBlocks, (int64_t)sm_count() * per_sm));
+  return JUBIK_OK;
 }
 
+template <typename T, int L1, int MODE, bool FWD>
+int launch_rows(RowK& k, size_t smem, bool pdl, cudaStream_t s) {
+  int64_t grid = 0;
+  JUBIK_TRY((row_grid<T, L1, MODE, FWD>(k, smem, &grid)));
+  k.base = (int)(k.item0 / grid * grid);
+  return sep_launch(k_sep_rows<T, L1, MODE, FWD>, dim3((unsigned)grid), row_threads(k), smem, pdl,
+                    s, "k_sep_rows", k);
+}
+
+// Kernel arguments of a launch.
 template <typename T, int L1>
-int dispatch_rows(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaStream_t s) {
-  RowK k{};
+int row_args(const Geom& g, SepMode mode, const SepRows& a, RowK& k, size_t& smem) {
   k.a = a;
   k.mode = mode;
   k.nx = g.nx;
@@ -674,19 +705,34 @@ int dispatch_rows(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaS
   k.rp = row_pairs(g.n, g.nx, k.seqs);
   const int pairs = (g.nx + 1) / 2;
   k.per = (pairs + k.rp - 1) / k.rp;
-  const int64_t items = (int64_t)a.planes * k.per;
+  if (!a.all_planes) k.a.all_planes = a.planes;  // one chunk
+  const int64_t items = (int64_t)k.a.all_planes * k.per;
   if (items > 0x7fffffffLL) {
     set_error("separable rows: too many image rows for one launch");
     return JUBIK_ERR_UNSUPPORTED;
   }
-  k.items = (int)items;
+  // (slabs and row spectra of a chunk are addressed by the planes of the whole image)
+  const size_t row = (size_t)a.plane0 * g.n * (g.P / 2) * sizeof(cx<T>);
+  if (a.slab) k.a.slab = (const char*)a.slab - row * ((size_t)k.height * k.nslab);
+  if (a.rows) k.a.rows = (char*)a.rows - row * (size_t)g.nx;
+  k.item0 = a.plane0 * k.per;
+  k.items = (a.plane0 + a.planes) * k.per;
+  k.grid_items = (int)items;
   k.late = a.slab_run == 1 ? std::max(0, (g.n - 1) * g.dx - g.sr_max) : 0;
   k.few = g.n <= k.seqs && (grad ? g.K : g.P) <= 4 * g.dx && (g.n - 1) * g.dx <= g.sc_max;
   const int64_t reach = sep_reach(g) + k.step;
   k.mul_dx = mulhi_divisor(g.dx, reach);
   k.mul_step = mulhi_divisor(k.step, reach);
   k.div_per = mulhi_divisor(k.per, items + 1);
-  const size_t smem = row_smem<T, L1>(g.n, g.ny, k.rp, k.seqs);
+  smem = row_smem<T, L1>(g.n, g.ny, k.rp, k.seqs);
+  return JUBIK_OK;
+}
+
+template <typename T, int L1>
+int dispatch_rows(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaStream_t s) {
+  RowK k{};
+  size_t smem = 0;
+  JUBIK_TRY((row_args<T, L1>(g, mode, a, k, smem)));
   switch (mode) {
     case SEP_SKY: return launch_rows<T, L1, SEP_SKY, true>(k, smem, pdl, s);
     case SEP_COT:
@@ -700,7 +746,37 @@ int dispatch_rows(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaS
   }
 }
 
+// Threads of the likelihood's launches, with or without the rows onward.
+template <typename T, int L1>
+int like_threads(const Geom& g, int64_t* threads) {
+  SepRows a;
+  a.planes = g.M * g.E;
+  RowK k{};
+  size_t smem = 0;
+  JUBIK_TRY((row_args<T, L1>(g, SEP_LIKE, a, k, smem)));
+  int64_t with = 0, without = 0;
+  JUBIK_TRY((row_grid<T, L1, SEP_LIKE, true>(k, smem, &with)));
+  JUBIK_TRY((row_grid<T, L1, SEP_LIKE, false>(k, smem, &without)));
+  *threads = std::max(with, without) * row_threads(k);
+  return JUBIK_OK;
+}
+
 }  // namespace
+
+template <typename T>
+int sep_like_threads_t(const Geom& g, int64_t* threads) {
+  switch (g.P) {
+    case 160: return like_threads<T, 10>(g, threads);
+    case 192: return like_threads<T, 12>(g, threads);
+    case 256: return like_threads<T, 16>(g, threads);
+    case 320: return like_threads<T, 20>(g, threads);
+    case 384: return like_threads<T, 24>(g, threads);
+    case 512: return like_threads<T, 32>(g, threads);
+    default: break;
+  }
+  set_error("separable rows do not cover P=%d", g.P);
+  return JUBIK_ERR_UNSUPPORTED;
+}
 
 template <typename T>
 int sep_rows_t(const Geom& g, SepMode mode, const SepRows& a, bool pdl, cudaStream_t s) {
