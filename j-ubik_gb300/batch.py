@@ -100,9 +100,14 @@ class ProblemBatch:
         return [p.response(x).double().cpu().numpy() for p, x in zip(self.plans, self.x)]
 
     def autotune(self, candidates: Sequence[str] = ("fused", "fused_unit", "plain"),
-                 reps: int = 5) -> Dict[int, str]:
+                 reps: int = 5, grouped: bool = False) -> Dict[int, str]:
         """Time each candidate path on the largest problem of every FFT side
-        and rebuild the plans with the fastest.  Needs the data set first."""
+        and rebuild the plans with the fastest.  Needs the data set first.
+
+        ``grouped`` times grouped passes of that problem, for a batch that
+        :meth:`group` follows: at FFT sides 160 and 192 a grouped pass runs the
+        fused kernels, a pass of one plan the separable ones.  Sides that no
+        candidate groups keep the times of one plan's passes."""
         if not hasattr(self, "_data"):
             raise RuntimeError("set_data before autotune")
         lib = _lib.load()
@@ -115,28 +120,10 @@ class ProblemBatch:
         for P, ks in sorted(by_side.items()):
             k = max(ks, key=lambda j: self.instruments[j].n_energies * self.instruments[j].shape[0]
                     * self.instruments[j].shape[1])
-            res = {}
-            for path in candidates:
-                if path != "plain" and not lib.jubik_fused_supported(P, code):
-                    continue
-                plan = self._make_plan(self.instruments[k], path)
-                try:
-                    plan.set_data(self._data[k])
-                    e = torch.empty((), dtype=torch.float64, device=self.device)
-                    g = torch.empty_like(self.x[k])
-                    for _ in range(2):
-                        plan.energy_and_grad(self.x[k], energy=e, grad=g)
-                    s = torch.cuda.current_stream(self.device)
-                    t0 = torch.cuda.Event(enable_timing=True)
-                    t1 = torch.cuda.Event(enable_timing=True)
-                    t0.record(s)
-                    for _ in range(reps):
-                        plan.energy_and_grad(self.x[k], energy=e, grad=g)
-                    t1.record(s)
-                    t1.synchronize()
-                    res[path] = t0.elapsed_time(t1) / reps
-                finally:
-                    plan.close()
+            paths = [p for p in candidates
+                     if p == "plain" or lib.jubik_fused_supported(P, code)]
+            res = self._time_paths(k, paths, reps, True) if grouped else {}
+            res = res or self._time_paths(k, paths, reps, False)
             best = min(res, key=res.get)
             # near ties go to the module-shared kernels: they do less work in all
             # (one sky spectrum per patch for all modules), which counts once the
@@ -149,17 +136,52 @@ class ProblemBatch:
         if chosen != {P: self.paths.get(P, "auto") for P in chosen}:
             self.paths.update(chosen)
             self._rebuild()
-        # the forward's run length (patches whose shared block rows meet in TMEM)
-        # on every plan that runs the module-shared FP32 kernels at FFT side 192
+        # the forward's run length (patches whose shared rows meet in TMEM) of every
+        # module-shared FP32 plan at FFT side 192: a setting of its own passes, which
+        # grouped ones do not use
         self.run_timings = {}
         for k, plan in enumerate(self.plans):
             if plan.shared_spectra and plan.dtype == torch.float32 and plan.P == 192:
                 self.run_timings[k] = plan.autotune(self.x[k], reps=reps)
         return chosen
 
+    def _time_paths(self, k: int, paths: Sequence[str], reps: int, grouped: bool
+                    ) -> Dict[str, float]:
+        """ms per pass of problem k alone on each path, grouped (paths that group) or not."""
+        res = {}
+        for path in paths:
+            one = ProblemBatch([self.instruments[k]], dtype=self.dtype,
+                               paths={_fft_side(self.instruments[k]): path}, device=self.device)
+            try:
+                one.set_data([self._data[k]])
+                if grouped and not one.group():
+                    continue
+                one.x[0].copy_(self.x[k])
+                for _ in range(2):
+                    one.energy_and_grad()
+                s = torch.cuda.current_stream(self.device)
+                t0 = torch.cuda.Event(enable_timing=True)
+                t1 = torch.cuda.Event(enable_timing=True)
+                t0.record(s)
+                for _ in range(reps):
+                    one.energy_and_grad()
+                t1.record(s)
+                t1.synchronize()
+                res[path] = t0.elapsed_time(t1) / reps
+            finally:
+                one.close()
+        return res
+
     def group(self) -> bool:
         """Switch the pass to grouped launches; False (and the per-problem pass
-        stays) when a problem takes the unfused path."""
+        stays) when a problem takes the unfused path.
+
+        Grouping pays where a problem by itself leaves the GPU idle.  At FFT sides
+        160 and 192 a grouped pass runs the fused kernels where one plan's pass runs
+        the separable ones: 64 fields of 128^2 take 0.12 ms grouped and 0.35 ms as a
+        captured loop, but two of 1024^2 x 7 x 3 take 2.8 and 1.6 ms, and eight of
+        256^2 x 7 x 3 0.74 and 0.49 ms (:meth:`capture`).  The two agree to FP32
+        rounding there, and to the last bits at the other sides."""
         self._drop_group()
         lib = _lib.load()
         n = len(self.plans)
