@@ -233,16 +233,6 @@ __device__ __forceinline__ void load_class(const cx<T>* h, cx<T> (&v)[16]) {
   for (int q = 0; q < 16; ++q)
     v[q] = PAST_L1 ? col_load_past_l1(h + q * (8 * L1)) : __ldg(h + q * (8 * L1));
 }
-// twiddles q and q + 1 (q even) of a class in one 16-byte load (FP32)
-__device__ __forceinline__ void two_twiddles(const float2* tw, int q, float2& a, float2& b) {
-  const float4 t = *reinterpret_cast<const float4*>(tw + q);
-  a = make_float2(t.x, t.y);
-  b = make_float2(t.z, t.w);
-}
-__device__ __forceinline__ void two_twiddles(const double2* tw, int q, double2& a, double2& b) {
-  a = tw[q];
-  b = tw[q + 1];
-}
 template <typename T, int L1>
 __device__ __forceinline__ void tile_to_spectrum(const cx<T>* t, const cx<T>* mytw, cx<T> (&v)[16]) {
 #pragma unroll

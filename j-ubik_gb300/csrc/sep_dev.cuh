@@ -36,6 +36,17 @@ __device__ __forceinline__ cx<T> split_b(cx<T> a, cx<T> b) {
   return mkc<T>(a.y + b.y, b.x - a.x);
 }
 
+// twiddles q and q + 1 (q even) of a class in one 16-byte load (FP32)
+__device__ __forceinline__ void two_twiddles(const float2* tw, int q, float2& a, float2& b) {
+  const float4 t = *reinterpret_cast<const float4*>(tw + q);
+  a = make_float2(t.x, t.y);
+  b = make_float2(t.z, t.w);
+}
+__device__ __forceinline__ void two_twiddles(const double2* tw, int q, double2& a, double2& b) {
+  a = tw[q];
+  b = tw[q + 1];
+}
+
 // s + e = a + b exactly, part by part (Knuth's TwoSum)
 template <typename C>
 __device__ __forceinline__ void two_sum(C a, C b, C& s, C& e) {

@@ -92,17 +92,6 @@ int row_seqs(const Geom& g) {
 __device__ __forceinline__ int row_div(int u, uint32_t mul) { return (int)__umulhi((uint32_t)u, mul); }
 __device__ __forceinline__ int row_slot(int z) { return (z >> 4) * 17 + (z & 15); }
 
-// twiddles q and q + 1 (q even) of a class in one 16-byte load (FP32)
-__device__ __forceinline__ void row_twiddles(const float2* tw, int q, float2& a, float2& b) {
-  const float4 t = *reinterpret_cast<const float4*>(tw + q);
-  a = make_float2(t.x, t.y);
-  b = make_float2(t.z, t.w);
-}
-__device__ __forceinline__ void row_twiddles(const double2* tw, int q, double2& a, double2& b) {
-  a = tw[q];
-  b = tw[q + 1];
-}
-
 // Writes p = a + i b at kx = lane + 32 t and conj m, m = a - i b, at P - kx of the pair's
 // sequence (kx = 0: the packed real kx = 0 and kx = P / 2 values of a and b).
 template <typename T, int L1>
@@ -351,7 +340,7 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
 #pragma unroll
             for (int q = 0; q < 16; q += 2) {
               cx<T> wa, wb;
-              row_twiddles(mytw, q, wa, wb);
+              two_twiddles(mytw, q, wa, wb);
               v[q] = q ? cmulc<T>(src[q], wa) : src[q];
               v[q + 1] = cmulc<T>(src[q + 1], wb);
             }
@@ -596,7 +585,7 @@ __global__ void __launch_bounds__(kRowThreads, row_ctas<T, L1>()) k_sep_rows(Row
 #pragma unroll
           for (int q = 0; q < 16; q += 2) {
             cx<T> wa, wb;
-            row_twiddles(mytw, q, wa, wb);
+            two_twiddles(mytw, q, wa, wb);
             dst[q] = q ? cmul<T>(v[q], wa) : v[q];
             dst[q + 1] = cmul<T>(v[q + 1], wb);
           }
