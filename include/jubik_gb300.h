@@ -187,8 +187,8 @@ JUBIK_API int jubik_plan_set_dependent_launch(jubik_plan* plan, int32_t on);
  * leave the CTA.  run_len 4 reduces fewest rows, 2 or 1 (one patch at a time)
  * give more work items for small fields; 0 (the default) lets the library
  * choose from the field size and the SM count.  Results agree to FP32 rounding
- * across run lengths and are the same bits for a given one.  Returns
- * JUBIK_ERR_UNSUPPORTED for runs the plan's geometry cannot take. */
+ * across run lengths and are the same bits for a given one.  Every plan takes 1;
+ * JUBIK_ERR_UNSUPPORTED for 2 and 4 on plans they are not a setting of. */
 JUBIK_API int jubik_plan_set_forward_run(jubik_plan* plan, int32_t run_len);
 /* The run length the plan's forward uses: the one set, or the library's choice. */
 JUBIK_API int jubik_plan_forward_run(const jubik_plan* plan, int32_t* run_len);

@@ -114,11 +114,12 @@ bool sep_run_fits(const Geom& g, int dtype, int run) {
 
 // Longer runs write fewer rows (6 strides per run of 4 patches, 12 without) and leave
 // fewer to sum, but make fewer CTAs.  The longest run is taken that still leaves 1.5
-// waves of CTAs, 2 with fewer than three modules, which have less to save.  A pass with
-// runs of 1 / 2 / 4, in us (waves of runs of 4): 1024^2 x 7 x 3 980 / 923 / 924 (3.8),
-// 1024^2 x 1 x 3 277 / 268 / 262 (3.8), 768^2 x 3 x 2 216 / 206 / 216 (1.4),
-// 512^2 x 7 x 3 283 / 270 / 283 (0.95), 1024^2 x 1 x 1 117 / 113 / 115 (1.3),
-// P = 384: 1024^2 x 7 x 3 1088 / 1070 / 1052 (3.8).
+// waves of CTAs, 2 with fewer than three modules.  A pass with runs of 1 / 2 / 4, in us
+// (waves of runs of 4): 1024^2 x 7 x 3 909 / 869 / 855 (3.8), 768^2 x 3 x 2 190 / 183 / 191
+// (1.4), 512^2 x 7 x 3 260 / 254 / 265 (0.95); of 1 and of the run taken: 1024^2 x 1 x 3
+// 241 / 225 (4; 3.8), 1024^2 x 1 x 1 97 / 95 (2; 1.3), P = 384 1024^2 x 7 x 3 970 / 875
+// (4; 3.8).  Few modules gain little: at 512^2 x 2 x 3 (1.9 waves of runs of 2) all lie
+// within 1.3 %, 104.3 / 103.7 / 105.1, so the line between 1 and 2 could lie on either side.
 int sep_auto_run(const Geom& g, int dtype) {
   const double least = g.M >= 3 ? 1.5 : 2.0;
   for (const int r : {4, 2})

@@ -58,3 +58,25 @@ def test_plans_without_runs_report_1(cuda):
             assert plan.set_forward_run(1).forward_run == 1
         finally:
             plan.close()
+
+
+# (field, modules, energies, the library's run): FFT side 192 in strides of 64 rows.  A CTA of
+# the forward's columns holds a run of patches and 8 of 96 columns, and an SM four CTAs; the
+# longest of 4 and 2 that makes 1.5 waves (2 with fewer than three modules) is taken.
+WAVES = [(1024, 7, 3, 4), (768, 3, 2, 2), (512, 7, 3, 2), (512, 2, 3, 1), (512, 3, 1, 1),
+         (1024, 2, 1, 2)]
+
+
+@pytest.mark.parametrize("geom", WAVES, ids=lambda g: "x".join(map(str, g)))
+def test_library_choice_follows_the_waves(cuda, geom):
+    nx, M, E, run = geom
+    n, sms = nx // 64, torch.cuda.get_device_properties(cuda).multi_processor_count
+    least = 1.5 if M >= 3 else 2.0
+    fits = [r for r in (4, 2) if E * n * (n // r) * 12 / (4.0 * sms) >= least]
+    if sms == 152:
+        assert (fits or [1])[0] == run
+    plan = ju.ResponsePlan(M, E, (nx, nx), n, 32, dtype=torch.float32)
+    try:
+        assert plan.forward_run == (fits or [1])[0]
+    finally:
+        plan.close()
