@@ -15,10 +15,10 @@
 // that 16 warps share an SM in independent CTAs: one CTA's loads overlap another's
 // transforms.  Within a CTA the PSF spectra (and the adjoint's rows) are loaded
 // into registers one transform ahead.  The kernels are bound by the LSU data
-// pipe (45-60 % busy: the exchange between the two phases, the twiddles, the
-// loads) together with instruction issue (about 55 %), beside DRAM: at
-// 1024^2 x 7 x 3 the forward moves 1298 MB in 284 us (4.6 TB/s), the adjoint
-// 1195 MB in 243 us (4.9 TB/s of a copy's 6.8); the per-patch kernels before
+// pipe (forward 47 %, adjoint 56 % busy at 512^2: the exchange between the two phases, the
+// twiddles, the loads) together with instruction issue (43 and 48 %), beside DRAM: at
+// 1024^2 x 7 x 3 the forward moves 1297 MB in 288 us (4.5 TB/s), the adjoint
+// 1194 MB in 243 us (4.9 TB/s of a copy's 6.8); the per-patch kernels before
 // them took 519 and 511 us.  The module sum stays in registers (250 us; 306 in
 // tensor memory); the rows that later patches of a run also cover wait in tensor
 // memory (TMEM, 128 lanes x 512 columns per SM, otherwise unused), which costs
